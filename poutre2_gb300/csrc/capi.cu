@@ -165,20 +165,42 @@ static pg_status repeat_small(const pg_image &in, int se, int iter, const pg_ima
 // Y segment).  Iterating the 3x3 square, or a 3-pixel X or Y segment, k times under the clipped
 // border equals one pass of the box k times as wide: along each axis every pixel between two
 // in-image pixels is in the image, so both reach the same pixels.  Whichever form is faster runs.
-// On 4096^2 images a 3-pixel pass costs 10-15 us (1-, 2-byte pixels), a line pass of any length
-// 20-30 us: the square runs as repeated 3x3 passes up to 4 (1-, 2-byte pixels) or 2 (wider),
-// a 3-pixel segment as one 3-pixel pass, anything else as line passes.
+//
+// Which form runs, with the times of a 4096^2 image (rows of whole 16-byte vectors) or a 2999 x 4001 one
+// (ragged rows) in us, the form not taken second:
+//   3-pixel passes (small_se.cu, small_tile.cu): 3x3 u8 10 / 22, f32 22 / 37; the square iterated twice from
+//     4 Mpixel on (u8 20 / 25, f32 2720 x 2912 23 / 26; one launch is better below: f32 1080 x 1920 window
+//     12 / 16), no further (u8 k = 3: window 27 / 28, k = 4: 25 / 36).  Ragged rows of a large image take the
+//     window kernel (window.cu) at once: 3x3 u8 19 / 35, X segment f32 27 / 37; below 3 Mpixel (4-byte
+//     pixels: 8, f32 2052 x 1674 13 / 11) its fixed cost weighs more (500 x 501: 8 / 6);
+//   k = 7, 15, 31 on 16-byte rows: the TMA tiles (Y segments diag.cu, boxes rect.cu): 31x31 u16 20 / 51;
+//   rectangles: the window kernel: u8 21x21 33 / 44, f32 11x11 53 / 95, ragged u8 29 / 120; where rows are
+//     whole words the two line passes win from hy + hx = 45 on (u8 45x45 46 / 46, 63x63 50 / 57);
+//   X segments: the word tiles (line_w.cu), where rows are whole words (u8 k = 10 20 / 22, u16 27 / 31), but
+//     the window kernel for short ones of 4-byte pixels (k = 2 35 / 45; k = 4 5024 x 5296 57 / 67 but 668 x
+//     4304 13 / 11; k = 10 47 / 45) and for ragged rows (u8 k = 10 20 / 61);
+//   Y segments: launch_line (line.cu).
 static pg_status box(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, bool dilate, cudaStream_t s) {
-  const int64_t square_passes_max = elem_size(in.ptype) <= 2 ? 4 : 2;
+  const int es = elem_size(in.ptype);
+  const bool words = rows_aligned(in, out, 4), vectors = rows_aligned(in, out, 16);
+  const bool window = window_ok(in, out, hy, hx, 0);
+  pg_status st = PG_OK;
+  const int64_t n = dims_of(in).count();
+  if (hx == 1 && hy <= 1 && !vectors && window && n >= (es <= 2 ? 3 << 20 : 8 << 20) &&
+      try_window(in, out, hy, hx, 0, dilate, s, &st))
+    return st;
   if (hy == 0 && hx == 1)
     return launch_small_se(in, out, in.rank == 1 ? PG_SE_SEGMENT_X_1D : PG_SE_SEGMENT_X_2D, dilate, s);
   if (in.rank == 2 && hy == 1 && hx == 0) return launch_small_se(in, out, PG_SE_SEGMENT_Y_2D, dilate, s);
+  const int64_t square_passes_max =
+      window ? (vectors && n >= (4 << 20) ? 2 : 1) : (es <= 2 ? 4 : 2);
   if (in.rank == 2 && hy == hx && hy >= 1 && hy <= square_passes_max)
     return repeat_small(in, PG_SE_SQUARE_2D, (int)hy, out, dilate, s);
-  pg_status st = PG_OK;
   // Y segment: the segment tile kernel (diag.cu), measured faster than the box tile for every type
   if (hx == 0 && hy <= 31 && try_segment_tile(in, out, 1, 0, (int)hy, dilate, s, &st)) return st;
   if (try_rect_fused(in, out, hy, hx, dilate, s, &st)) return st;  // shared-memory tile pass (rect.cu)
+  const bool best = hy == 0 ? !words || (es == 4 && hx <= (n >= (8 << 20) ? 5 : 3)) : hx > 0 && (!words || hy + hx <= 44);
+  if (window && best && try_window(in, out, hy, hx, 0, dilate, s, &st)) return st;
   if (hy == 0) return launch_line(in, out, 0, 1, hx, dilate, s);
   return launch_rect(in, out, hy, hx, dilate, s);
 }

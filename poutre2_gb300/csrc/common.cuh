@@ -248,6 +248,12 @@ inline Dims dims_of(const pg_image &im) {
   return d;
 }
 
+// both images' rows start on multiples of `unit` bytes
+inline bool rows_aligned(const pg_image &in, const pg_image &out, int unit) {
+  return (dims_of(in).nx * elem_size(in.ptype)) % unit == 0 &&
+         (reinterpret_cast<uintptr_t>(in.data) | reinterpret_cast<uintptr_t>(out.data)) % (uintptr_t)unit == 0;
+}
+
 // ------------------------------------------------------------------ kernel entry points
 // (host launchers, implemented in the .cu files)
 pg_status launch_small_se(const pg_image &in, const pg_image &out, int se, bool dilate, cudaStream_t s);
@@ -277,6 +283,12 @@ int take_oct_status();  // device status of the octagon tile kernel since the la
 // rows of a multiple of 16 bytes.
 bool try_small_tile(const pg_image &in, const pg_image &out, int se, bool dilate, cudaStream_t s, pg_status *st);
 int take_small_tile_status();  // device status of the small-SE tile kernel since the last call (0: none)
+// Boxes and vertical / 45- / 135-degree segments (lean = the pixels a row moves right per row: hx = 0) of any
+// half lengths up to 63 (row windows of at most half a tile row), any row length and alignment (window.cu):
+// 1-, 2- and 4-byte pixels, images of at least 16 rows.
+bool window_ok(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, int lean);
+bool try_window(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, int lean, bool dilate, cudaStream_t s,
+                pg_status *st);
 pg_status launch_rect(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, bool dilate, cudaStream_t s);
 // One-pass box (rect.cu): (hy, hx) = (k, k), (0, k) or (k, 0), k in {7, 15, 31}; 2-/4-byte pixels,
 // rows of a multiple of 16 bytes.  try_rect_gradient: dilation - erosion in the same pass.

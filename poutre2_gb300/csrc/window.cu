@@ -1,0 +1,426 @@
+// window.cu -- erosion / dilation of 2D images by a (2hy+1) x (2hx+1) box or by a vertical / 45- / 135-degree
+// segment of any half length, for 1-, 2- and 4-byte pixels, rows of any length and alignment, in one pass.
+//
+// Same result as line.cu / line_w.cu (X then Y van Herk passes, ero_dil_line_se_t.hpp:50-89, clipped
+// windows; the diagonals are the runtime neighbour-list segments); the half lengths are run-time values.
+// The window extremum is built from windows of fixed lengths (along rows powers of two, each from two of half
+// the length): a handful of steps whatever the window, none of which needs its length at compile time, where
+// a van Herk scan keeps a window of registers per thread.
+//
+// A CTA (8 warps) owns a tile of up to 120 32-bit words (E = 4 / sizeof(T) pixels each) x TH rows:
+//   rows    -- a warp takes a row of 128 words (a lane 4 consecutive words).  The row starts hx pixels left
+//              of the tile at any byte: aligned words are loaded and funnel-shifted.  Forward windows of
+//              length 2hx + 1 are put together in registers along the binary expansion of the length; the
+//              shifts are powers of two, inside a lane's words or whole lanes (shuffles).  u8 pixels are
+//              kept as even / odd pixels on 16-bit lanes (two max.u16x2 per word; the packed 4 x 8-bit
+//              instruction is an emulated sequence on this GPU).  The result goes to shared memory.
+//   columns -- a thread walks up its word column and replaces each word by the window of 3 or 9 rows
+//              (delay lines in registers, one shared load and store per word; three values meet in one
+//              instruction); then
+//   output  -- every output is the extremum of ceil((2hy+1) / 9) of those, and is shifted to the
+//              alignment of its row in memory by one shuffle, so that stores are whole aligned words.
+// A diagonal segment is a column of a sheared tile: row y of the tile starts lean * (y - y0) pixels further
+// right, which the unaligned loads and stores absorb.
+//
+// Bound: the ALU pipe (min / max, shifts and byte permutes all issue there at half rate; 54 % busy at 2999 x
+// 4001 u8, 21x21) and the waits of the 24 warps an image of that size gives an SM; the input is read from
+// DRAM once, the halo from L2.  2999 x 4001 u8: 21x21 120 -> 29 us, 45-degree segment of 21 90 -> 21 us (pixel-
+// wise van Herk in shared memory before: rows of no whole words); f32 4096^2 45 degrees of 21 104 -> 43 us.
+#include <algorithm>
+#include <atomic>
+
+#include "common.cuh"
+#include "words.cuh"
+
+namespace pg {
+namespace {
+
+constexpr int kWThreads = 256, kWWarps = kWThreads / 32;
+constexpr int kWRow = 128;                       // words of a tile row
+constexpr int kWOut = 4 * 31;                    // words the four warps of a column pass put out (lane 0 lends)
+constexpr size_t kWSmemMax = 227 * 1024;
+
+// A word as the operands of the min / max instructions: u8 words as two words whose 16-bit lanes hold the
+// even / odd pixels in their high byte (the low byte only breaks ties), others as they are.
+template <typename T, bool SUP> struct Acc {
+  static constexpr bool B8 = sizeof(T) == 1;
+  uint32_t a, b;
+  __device__ __forceinline__ static uint32_t op16(uint32_t x, uint32_t y) { return wop<uint16_t, SUP>(x, y); }
+  __device__ __forceinline__ static Acc of(uint32_t w) {
+    if constexpr (B8) return Acc{w << 8, w};
+    else return Acc{w, 0u};
+  }
+  __device__ __forceinline__ Acc with(const Acc &o) const {
+    if constexpr (B8) return Acc{op16(a, o.a), op16(b, o.b)};
+    else return Acc{wop<T, SUP>(a, o.a), 0u};
+  }
+  __device__ __forceinline__ uint32_t word() const {
+    if constexpr (B8) return __byte_perm(a, b, 0x7351);
+    else return a;
+  }
+};
+
+// A lane's four words of a row in registers, as NR registers of two 16-bit lanes or one 32-bit pixel:
+// u8: r[2j] = even, r[2j + 1] = odd pixels of word j (clean 16-bit lanes); others: r[j] = word j.
+template <typename T> struct RowRegs {
+  static constexpr int NR = sizeof(T) == 1 ? 8 : 4;
+  uint32_t r[NR];
+  __device__ __forceinline__ static RowRegs of(const uint32_t (&w)[4]) {
+    RowRegs o;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if constexpr (sizeof(T) == 1) {
+        o.r[2 * j] = __byte_perm(w[j], 0u, 0x4240);
+        o.r[2 * j + 1] = __byte_perm(w[j], 0u, 0x4341);
+      } else {
+        o.r[j] = w[j];
+      }
+    }
+    return o;
+  }
+  __device__ __forceinline__ uint4 words() const {
+    if constexpr (sizeof(T) == 1)
+      return make_uint4(__byte_perm(r[0], r[1], 0x6240), __byte_perm(r[2], r[3], 0x6240),
+                        __byte_perm(r[4], r[5], 0x6240), __byte_perm(r[6], r[7], 0x6240));
+    else
+      return make_uint4(r[0], r[1], r[2], r[3]);
+  }
+};
+
+__device__ __forceinline__ uint32_t from_lane(uint32_t v, int ahead) { return __shfl_down_sync(0xffffffffu, v, ahead); }
+
+// the row moved left by S pixels (a power of two): pixel i takes pixel i + S.  The last lanes take
+// anything; they feed no output.
+template <typename T, int S> __device__ __forceinline__ RowRegs<T> ahead(const RowRegs<T> &x) {
+  constexpr int E = 4 / (int)sizeof(T), LP = 4 * E, NR = RowRegs<T>::NR;  // pixels per word, per lane
+  RowRegs<T> o;
+  if constexpr (S >= LP) {
+#pragma unroll
+    for (int j = 0; j < NR; ++j) o.r[j] = from_lane(x.r[j], S / LP);
+  } else if constexpr (S >= E) {  // whole words
+    constexpr int D = S / E * (NR / 4);
+#pragma unroll
+    for (int j = 0; j < NR; ++j) o.r[j] = j + D < NR ? x.r[j + D] : from_lane(x.r[j + D - NR], 1);
+  } else if constexpr (sizeof(T) == 2) {  // S = 1
+    const uint32_t n = from_lane(x.r[0], 1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o.r[j] = __funnelshift_r(x.r[j], j < 3 ? x.r[j + 1] : n, 16);
+  } else if constexpr (S == 1) {  // u8: the odd pixels, and the even ones from the next on
+    const uint32_t n = from_lane(x.r[0], 1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      o.r[2 * j] = x.r[2 * j + 1];
+      o.r[2 * j + 1] = __funnelshift_r(x.r[2 * j], j < 3 ? x.r[2 * j + 2] : n, 16);
+    }
+  } else {  // u8, S = 2
+    const uint32_t n0 = from_lane(x.r[0], 1), n1 = from_lane(x.r[1], 1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      o.r[2 * j] = __funnelshift_r(x.r[2 * j], j < 3 ? x.r[2 * j + 2] : n0, 16);
+      o.r[2 * j + 1] = __funnelshift_r(x.r[2 * j + 1], j < 3 ? x.r[2 * j + 3] : n1, 16);
+    }
+  }
+  return o;
+}
+template <typename T, bool SUP> __device__ __forceinline__ RowRegs<T> both(const RowRegs<T> &x, const RowRegs<T> &y) {
+  RowRegs<T> o;
+#pragma unroll
+  for (int j = 0; j < RowRegs<T>::NR; ++j)
+    o.r[j] = sizeof(T) == 1 ? wop<uint16_t, SUP>(x.r[j], y.r[j]) : wop<T, SUP>(x.r[j], y.r[j]);
+  return o;
+}
+
+// forward windows of w pixels (w odd, below 2^7), along w's bits: m holds windows of 2^j, res those of the
+// bits so far
+template <typename T, bool SUP, int J>
+__device__ __forceinline__ void row_steps(RowRegs<T> &m, RowRegs<T> &res, int w) {
+  if (w >> J) {  // uniform; m: windows of 2^(J-1) -> 2^J
+    m = both<T, SUP>(m, ahead<T, 1 << (J - 1)>(m));
+    if ((w >> J) & 1) res = both<T, SUP>(m, ahead<T, 1 << J>(res));
+    if constexpr (J < 6) row_steps<T, SUP, J + 1>(m, res, w);
+  }
+}
+
+struct WindowGeom {
+  int64_t H, W;
+  int hx;          // half width
+  int hy;          // half height
+  int lean;        // pixels a tile row starts further right than the row above: -1, 0, 1
+  int th;          // output rows of a tile, a multiple of 8
+  int half;        // half the rows of the tile's array in shared memory, a multiple of 6
+  int vw;          // output words of a tile row
+  int64_t u_first; // first pixel of tile column 0 at the tile's first output row
+};
+
+// Columns, in place: word of row i <- op over rows [i, i + N), N = 3 or 9 (the min / max of three values is
+// one instruction).  Group [ga, ga + half) of the 2 * half rows of the tile's array, walking up (half a
+// multiple of 6); the N - 1 rows below the first group prime its delay lines before any is overwritten.
+// Rows past the tile's last only reach windows no output uses.
+template <typename T, bool SUP, int N>
+__device__ __forceinline__ void column_windows(uint32_t *col, int ga, int half) {
+  using A = Acc<T, SUP>;
+  constexpr int B = 6;  // steps per unrolled turn: every delay line's length divides it
+  const A neu = A::of(splat<T>(Op<T, SUP>::neutral()));
+  A d1[2] = {neu, neu}, d3[6] = {neu, neu, neu, neu, neu, neu};
+  auto step = [&](A x, int i) -> A {
+    A m = x.with(d1[0]).with(d1[1]);  // rows r .. r + 2
+    d1[i % 2] = x;
+    if constexpr (N == 9) {
+      const A t = m.with(d3[i % 6]).with(d3[(i + 3) % 6]);  // the windows 6 and 3 rows below
+      d3[i % 6] = m;
+      m = t;
+    }
+    return m;
+  };
+  if (ga == 0) {
+#pragma unroll
+    for (int i = 0; i < N - 1; ++i) {
+      const int r = half + N - 2 - i;
+      step(r < 2 * half ? A::of(col[r * kWRow]) : neu, i % B);
+    }
+  }
+  __syncthreads();
+  for (int r0 = ga + half - B; r0 >= ga; r0 -= B) {
+    uint32_t *q = col + r0 * kWRow, x[B];
+#pragma unroll
+    for (int i = 0; i < B; ++i) x[i] = q[(B - 1 - i) * kWRow];
+#pragma unroll
+    for (int i = 0; i < B; ++i) q[(B - 1 - i) * kWRow] = step(A::of(x[i]), (i + N - 1) % B).word();
+  }
+}
+
+// This lane's four words from the aligned address of row byte `a` on, for a row of words that may reach
+// beyond the image's bytes [base, end): the bytes of a word across an end come one by one.
+__device__ __noinline__ uint4 edge_words(uintptr_t a, uintptr_t base, uintptr_t end) {
+  const uintptr_t p = (a & ~(uintptr_t)3) + 16u * (threadIdx.x & 31);
+  uint32_t w[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uintptr_t pw = p + 4u * j;
+    w[j] = 0u;
+    if (pw >= base && pw + 4 <= end) {
+      w[j] = __ldg(reinterpret_cast<const uint32_t *>(pw));
+    } else {
+      for (int b = 0; b < 4; ++b)
+        if (pw + b >= base && pw + b < end)
+          w[j] |= (uint32_t)*reinterpret_cast<const unsigned char *>(pw + b) << (8 * b);
+    }
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+template <typename T, bool SUP>
+__global__ void __launch_bounds__(kWThreads) k_window(const T *__restrict__ in, T *__restrict__ out, WindowGeom g) {
+  constexpr int S = (int)sizeof(T), E = 4 / S;
+  extern __shared__ __align__(16) uint32_t s_w[];  // [2 * half][kWRow]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t NEU = splat<T>(Op<T, SUP>::neutral());
+  const int64_t u0 = g.u_first + (int64_t)blockIdx.x * g.vw * E;  // the tile's first pixel in its first output row
+  const int64_t y0 = (int64_t)blockIdx.y * g.th;
+  const int rows = g.th + 2 * g.hy, half = g.half;
+  const intptr_t pitch = (intptr_t)(g.W + g.lean) * S;  // bytes from a tile row to the next
+
+  // ---- rows, two at a time per warp so that the loads of both are in flight
+  {
+    // tile rows [r_lo, r_hi) are rows of the image
+    const int r_lo = (int)max((int64_t)0, g.hy - y0), r_hi = (int)min((int64_t)rows, g.H - y0 + g.hy);
+    // first pixel of tile row 0: one word left of the tile, for the stores' shift
+    const int64_t x_top = u0 - E - g.hx - (int64_t)g.lean * g.hy;
+    const int64_t x_bot = x_top + (int64_t)g.lean * (rows - 1);
+    const uintptr_t a_top = reinterpret_cast<uintptr_t>(in) + (uintptr_t)(((y0 - g.hy) * g.W + x_top) * S);
+    uintptr_t a = a_top + warp * pitch;
+    // some row holds pixels left / right of the image
+    const bool clipped = min(x_top, x_bot) < 0 || max(x_top, x_bot) + kWRow * E > g.W;
+    const uintptr_t base = reinterpret_cast<uintptr_t>(in), end = base + (uintptr_t)(g.H * g.W) * S;
+    // every row of words lies in the image's buffer
+    const bool safe = ((a_top + r_lo * pitch) & ~(uintptr_t)3) >= base && a_top + (r_hi - 1) * pitch + kWRow * 4 <= end;
+    const int wlen = 2 * g.hx + 1;
+    for (int r0 = warp; r0 < rows; r0 += 2 * kWWarps, a += 2 * kWWarps * pitch) {
+      uint32_t w[2][4];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int r = r0 + q * kWWarps;
+        const uintptr_t aq = a + q * kWWarps * pitch, seg = aq & ~(uintptr_t)3;
+        if (r < r_lo || r >= r_hi) continue;
+        if (safe || (seg >= base && seg + kWRow * 4 <= end)) {
+          const uintptr_t p = seg + 16u * lane;  // this lane's words
+          if ((aq & 12u) == 0) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
+            w[q][0] = v.x; w[q][1] = v.y; w[q][2] = v.z; w[q][3] = v.w;
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w[q][j] = __ldg(reinterpret_cast<const uint32_t *>(p) + j);
+          }
+        } else {
+          const uint4 v = edge_words(aq, base, end);
+          w[q][0] = v.x; w[q][1] = v.y; w[q][2] = v.z; w[q][3] = v.w;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int r = r0 + q * kWWarps;
+        if (r >= rows) break;
+        if (r < r_lo || r >= r_hi) {
+          *reinterpret_cast<uint4 *>(s_w + r * kWRow + lane * 4) = make_uint4(NEU, NEU, NEU, NEU);
+          continue;
+        }
+        const unsigned sh = (unsigned)((a + q * kWWarps * pitch) & 3u) * 8u;
+        if (S < 4 && sh) {
+          // the last word of lane 31 lacks its upper pixels: no output of the tile needs them (vw)
+          const uint32_t n = from_lane(w[q][0], 1);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) w[q][j] = __funnelshift_r(w[q][j], j < 3 ? w[q][j + 1] : n, sh);
+        }
+        if (clipped) {
+          // the lane's pixels [lo, hi) lie in the image
+          const int64_t x = x_top + (int64_t)g.lean * r + lane * 4 * E;
+          const int lo = (int)min(max(-x, (int64_t)0), (int64_t)4 * E), hi = (int)min(max(g.W - x, (int64_t)0), (int64_t)4 * E);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int l = min(max(lo - j * E, 0), E), k = min(max(hi - j * E, 0), E);  // of word j
+            const uint32_t in_m = (uint32_t)(((1ull << (8 * S * k)) - 1ull) & ~((1ull << (8 * S * l)) - 1ull));
+            w[q][j] = (w[q][j] & in_m) | (NEU & ~in_m);
+          }
+        }
+        uint4 o = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+        if (wlen > 1) {
+          RowRegs<T> m = RowRegs<T>::of(w[q]), res = m;
+          row_steps<T, SUP, 1>(m, res, wlen);
+          o = res.words();
+        }
+        *reinterpret_cast<uint4 *>(s_w + r * kWRow + lane * 4) = o;
+      }
+    }
+  }
+  __syncthreads();
+
+  // ---- columns: four warps side by side, two groups of rows
+  const int h = 2 * g.hy + 1;
+  int n = 1;  // window length left in shared memory
+  if (h >= 5) {
+    uint32_t *mine = s_w + (threadIdx.x & (kWRow - 1));
+    const int ga = (threadIdx.x >> 7) * half;
+    if (h < 9) { column_windows<T, SUP, 3>(mine, ga, half); n = 3; }
+    else { column_windows<T, SUP, 9>(mine, ga, half); n = 9; }
+    __syncthreads();
+  }
+  // ---- output: th / 2 rows per group (a multiple of 4)
+  using A = Acc<T, SUP>;
+  // Word column c of the tile lies at array column c + 1; with its row's alignment it covers the pixels from
+  // c * E - (pixels past an aligned word) on, so every word is stored whole but at the image's sides.
+  const int c = (warp & 3) * 31 + lane - 1;  // lane 0 only lends its word to lane 1
+  const int gh = g.th / 2, ya = (warp >> 2) * gh;
+  const int yb = (int)min((int64_t)(ya + gh), g.H - y0);
+  const int64_t x_end = u0 + (int64_t)g.lean * (g.th - 1);
+  const bool inner = min(u0, x_end) >= E && max(u0, x_end) + g.vw * E <= g.W;
+  const bool mine = lane > 0 && c < g.vw;
+  const uint32_t *q = s_w + c + 1 + ya * kWRow;
+  uintptr_t a = reinterpret_cast<uintptr_t>(out) + (uintptr_t)(((y0 + ya) * g.W + u0 + (int64_t)g.lean * ya) * S);
+  constexpr int U = 4;
+  for (int y = ya; y < yb; y += U, q += U * kWRow, a += U * pitch) {
+    A v[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) v[k] = A::of(q[k * kWRow]);
+    if (h > n) {
+      const uint32_t *qt = q + n * kWRow, *ql = q + (h - n) * kWRow;
+      for (; qt + n * kWRow < ql; qt += 2 * n * kWRow)  // two windows at a time: one instruction takes both
+#pragma unroll
+        for (int k = 0; k < U; ++k) v[k] = v[k].with(A::of(qt[k * kWRow])).with(A::of(qt[(n + k) * kWRow]));
+      if (qt < ql)
+#pragma unroll
+        for (int k = 0; k < U; ++k) v[k] = v[k].with(A::of(qt[k * kWRow])).with(A::of(ql[k * kWRow]));
+      else
+#pragma unroll
+        for (int k = 0; k < U; ++k) v[k] = v[k].with(A::of(ql[k * kWRow]));
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (y + k >= yb) break;  // uniform
+      const uintptr_t ak = a + k * pitch;
+      const unsigned mis = S < 4 ? (unsigned)(ak & 3u) : 0u;  // bytes past an aligned word
+      uint32_t o = v[k].word();
+      if (mis) o = __funnelshift_l(__shfl_up_sync(0xffffffffu, o, 1), o, mis * 8u);
+      if (!mine) continue;
+      T *dst = reinterpret_cast<T *>((ak & ~(uintptr_t)3) + 4 * (intptr_t)c);
+      if (inner) {
+        *reinterpret_cast<uint32_t *>(dst) = o;
+      } else {
+        const int64_t x = u0 + (int64_t)g.lean * (y + k) + c * E - (int)mis / S;  // the word's first pixel
+        if (x >= 0 && x + E <= g.W) {
+          *reinterpret_cast<uint32_t *>(dst) = o;
+        } else if (S < 4 && x + E > 0 && x < g.W) {
+#pragma unroll
+          for (int e = 0; e < E; ++e)
+            if (x + e >= 0 && x + e < g.W) dst[e] = (T)(o >> (8 * S * e));
+        }
+      }
+    }
+  }
+}
+
+template <typename T, bool SUP>
+pg_status window_t(const pg_image &in, const pg_image &out, WindowGeom g, cudaStream_t s) {
+  constexpr int E = 4 / (int)sizeof(T);
+  // valid words of a row (windows are forward), in whole 32-byte sectors: a misaligned load loses a word, the
+  // stores' shift needs one left of the tile
+  g.vw = std::min((kWRow * E - 2 * g.hx) / E - 2, kWOut) & ~7;
+  // pixels a tile row has to reach beyond the image: the shear's, and a misaligned last word's
+  const bool mis = E > 1 && (g.lean != 0 || (g.W % E) != 0 || reinterpret_cast<uintptr_t>(out.data) % 4 != 0);
+  // 64 rows per tile, fewer (but no less than the halo's 2 hy) where the image would not give every SM four
+  // CTAs: 2999 x 4001 u8 3x3 20.5 -> 18.9 us with 32 rows, 21x21 28.7 with both
+  g.th = 64;
+  const int64_t sms = num_sms();
+  auto tiles_x = [&]() { return ceil_div(g.W + (g.lean ? g.th - 1 : 0) + (mis ? E - 1 : 0), (int64_t)g.vw * E); };
+  while (g.th > 16 && g.th / 2 >= 2 * g.hy && tiles_x() * ceil_div(g.H, g.th) < 4 * sms) g.th /= 2;
+  if (tiles_x() * ceil_div(g.H, g.th) < sms) g.th /= 2;  // 64, 32, 16 or 8: a group's rows are a multiple of 4
+  g.u_first = g.lean > 0 ? -(int64_t)(g.th - 1) : 0;
+  g.half = (g.th + 2 * g.hy + 11) / 12 * 6;
+  const size_t smem = (size_t)(2 * g.half) * kWRow * 4;
+  static std::atomic<uint64_t> attr_devices{0};
+  int dev = 0;
+  PG_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
+  const uint64_t bit = 1ull << (dev & 63);
+  if (!(attr_devices.load() & bit)) {
+    PG_CUDA_TRY(cudaFuncSetAttribute(k_window<T, SUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWSmemMax),
+                "window kernel smem attribute");
+    attr_devices.fetch_or(bit);
+  }
+  const dim3 grid((unsigned)tiles_x(), (unsigned)ceil_div(g.H, g.th));
+  k_window<T, SUP><<<grid, kWThreads, smem, s>>>(static_cast<const T *>(in.data), static_cast<T *>(out.data), g);
+  return cuda_status(cudaGetLastError(), "window kernel launch");
+}
+
+}  // namespace
+
+bool window_ok(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, int lean) {
+  const int es = elem_size(in.ptype);
+  if (in.rank != 2 || (es != 1 && es != 2 && es != 4)) return false;
+  if (hy < 0 || hx < 0 || hy > 63 || (hy == 0 && hx == 0) || (lean != 0 && hx != 0)) return false;
+  // a row window needs its length below 2^7 and leaves at least half of a tile row's pixels
+  if (hx > 63 || 4 * hx > kWRow * 4 / es) return false;
+  const Dims d = dims_of(in);
+  if (d.ny < 16 || d.nx < 1 || d.ny > (1 << 19) || d.nx > (1 << 30)) return false;
+  const uintptr_t pixel = (uintptr_t)es - 1;
+  return ((reinterpret_cast<uintptr_t>(in.data) | reinterpret_cast<uintptr_t>(out.data)) & pixel) == 0;
+}
+
+bool try_window(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, int lean, bool dilate, cudaStream_t s,
+                pg_status *st) {
+  if (!window_ok(in, out, hy, hx, lean)) return false;
+  const Dims d = dims_of(in);
+  WindowGeom g{};
+  g.H = d.ny;
+  g.W = d.nx;
+  g.hx = (int)hx;
+  g.hy = (int)hy;
+  g.lean = lean;
+  switch (in.ptype) {
+    case PG_PTYPE_U8: *st = dilate ? window_t<uint8_t, true>(in, out, g, s) : window_t<uint8_t, false>(in, out, g, s); return true;
+    case PG_PTYPE_U16: *st = dilate ? window_t<uint16_t, true>(in, out, g, s) : window_t<uint16_t, false>(in, out, g, s); return true;
+    case PG_PTYPE_I32: *st = dilate ? window_t<int32_t, true>(in, out, g, s) : window_t<int32_t, false>(in, out, g, s); return true;
+    case PG_PTYPE_F32: *st = dilate ? window_t<float, true>(in, out, g, s) : window_t<float, false>(in, out, g, s); return true;
+    default: return false;
+  }
+}
+
+}  // namespace pg
