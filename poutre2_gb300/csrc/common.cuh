@@ -289,6 +289,10 @@ int take_small_tile_status();  // device status of the small-SE tile kernel sinc
 bool window_ok(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, int lean);
 bool try_window(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, int lean, bool dilate, cudaStream_t s,
                 pg_status *st);
+// Neighbour lists through their chords, runs of offsets along a row (window.cu): 1-, 2- and 4-byte pixels, rank 2
+// and 3, at least 16 rows, lists whose chords are few for their offsets.
+bool try_chords(const pg_image &in, const pg_image &out, const int32_t *offsets, int n, bool dilate, cudaStream_t s,
+                pg_status *st);
 pg_status launch_rect(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, bool dilate, cudaStream_t s);
 // One-pass box (rect.cu): (hy, hx) = (k, k), (0, k) or (k, 0), k in {7, 15, 31}; 2-/4-byte pixels,
 // rows of a multiple of 16 bytes.  try_rect_gradient: dilation - erosion in the same pass.

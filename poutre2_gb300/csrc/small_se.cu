@@ -210,7 +210,8 @@ __global__ void __launch_bounds__(256) k_small3d(const T *__restrict__ in, T *__
   }
 }
 
-// Arbitrary neighbour list, gather form with border clipping.
+// Arbitrary neighbour list, gather form with border clipping: lists of few or scattered offsets, 8-byte pixels,
+// images of less than 16 rows (others by chords, window.cu).
 template <typename T, bool SUP>
 __global__ void __launch_bounds__(256) k_nl(const T *__restrict__ in, T *__restrict__ out, int64_t D, int64_t H,
                                             int64_t W, const int4 *__restrict__ offs, int n) {
@@ -341,6 +342,8 @@ pg_status launch_nl(const pg_image &in, const pg_image &out, const int32_t *offs
                     cudaStream_t s) {
   const Dims d = dims_of(in);
   if (d.count() == 0) return PG_OK;
+  pg_status st = PG_OK;
+  if (try_chords(in, out, offsets, n, dilate, s, &st)) return st;
   // offsets -> (dz, dy, dx, 0) int4 in device memory.  The host copy is pageable: the
   // runtime stages it before cudaMemcpyAsync returns, so it may be released right away.
   Scratch dev;

@@ -130,13 +130,13 @@ template <typename T, bool SUP> __device__ __forceinline__ RowRegs<T> both(const
   return o;
 }
 
-// forward windows of w pixels (w odd, below 2^7), along w's bits: m holds windows of 2^j, res those of the
-// bits so far
+// forward windows of w pixels (1 <= w < 2^7), along w's bits: m holds windows of 2^j, res those of the bits
+// so far (w odd: it starts as the pixels themselves; w even: it is set at w's lowest bit)
 template <typename T, bool SUP, int J>
 __device__ __forceinline__ void row_steps(RowRegs<T> &m, RowRegs<T> &res, int w) {
   if (w >> J) {  // uniform; m: windows of 2^(J-1) -> 2^J
     m = both<T, SUP>(m, ahead<T, 1 << (J - 1)>(m));
-    if ((w >> J) & 1) res = both<T, SUP>(m, ahead<T, 1 << J>(res));
+    if ((w >> J) & 1) res = (w & ((1 << J) - 1)) ? both<T, SUP>(m, ahead<T, 1 << J>(res)) : m;
     if constexpr (J < 6) row_steps<T, SUP, J + 1>(m, res, w);
   }
 }
@@ -209,89 +209,131 @@ __device__ __noinline__ uint4 edge_words(uintptr_t a, uintptr_t base, uintptr_t 
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// Stores a tile's output words, lane by lane word column c (c = -1 and lane 0 only lend): with its row's
+// alignment word c covers the pixels from c * E - (pixels past an aligned word) on, so that every word is
+// stored whole but at the image's sides.
+template <typename T> struct TileStore {
+  static constexpr int S = (int)sizeof(T), E = 4 / S;
+  int64_t W, u0;
+  int lean, c;
+  bool inner, mine;
+  __device__ __forceinline__ TileStore(int64_t W_, int64_t u0_, int lean_, int th, int vw, int c_)
+      : W(W_), u0(u0_), lean(lean_), c(c_) {
+    const int64_t x_end = u0 + (int64_t)lean * (th - 1);
+    inner = min(u0, x_end) >= E && max(u0, x_end) + vw * E <= W;
+    mine = (threadIdx.x & 31) != 0 && c < vw;
+  }
+  // word w of tile row y, whose pixel u0 + lean * y lies at byte address a; called by the whole warp
+  __device__ __forceinline__ void put(uintptr_t a, int y, uint32_t w) const {
+    const unsigned mis = S < 4 ? (unsigned)(a & 3u) : 0u;  // bytes past an aligned word
+    if (mis) w = __funnelshift_l(__shfl_up_sync(0xffffffffu, w, 1), w, mis * 8u);
+    if (!mine) return;
+    T *dst = reinterpret_cast<T *>((a & ~(uintptr_t)3) + 4 * (intptr_t)c);
+    if (inner) {
+      *reinterpret_cast<uint32_t *>(dst) = w;
+    } else {
+      const int64_t x = u0 + (int64_t)lean * y + c * E - (int)mis / S;  // the word's first pixel
+      if (x >= 0 && x + E <= W) {
+        *reinterpret_cast<uint32_t *>(dst) = w;
+      } else if (S < 4 && x + E > 0 && x < W) {
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+          if (x + e >= 0 && x + e < W) dst[e] = (T)(w >> (8 * S * e));
+      }
+    }
+  }
+};
+
+// Rows [0, rows) of a tile: row r starts at pixel x_top + lean * r of image row y_top + r; its words go to
+// s_w[r][..] as forward windows of wlen pixels, those outside the image neutral.  Two rows at a time per warp,
+// so that the loads of both are in flight.
+template <typename T, bool SUP>
+__device__ __forceinline__ void window_rows(const T *in, int64_t H, int64_t W, int64_t y_top, int64_t x_top, int lean,
+                                            int rows, int wlen, uint32_t *s_w) {
+  constexpr int S = (int)sizeof(T), E = 4 / S;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t NEU = splat<T>(Op<T, SUP>::neutral());
+  const intptr_t pitch = (intptr_t)(W + lean) * S;  // bytes from a tile row to the next
+  // tile rows [r_lo, r_hi) are rows of the image
+  const int r_lo = (int)min(max((int64_t)0, -y_top), (int64_t)rows), r_hi = (int)min((int64_t)rows, H - y_top);
+  const int64_t x_bot = x_top + (int64_t)lean * (rows - 1);
+  const uintptr_t a_top = reinterpret_cast<uintptr_t>(in) + (uintptr_t)((y_top * W + x_top) * S);
+  uintptr_t a = a_top + warp * pitch;
+  // some row holds pixels left / right of the image
+  const bool clipped = min(x_top, x_bot) < 0 || max(x_top, x_bot) + kWRow * E > W;
+  const uintptr_t base = reinterpret_cast<uintptr_t>(in), end = base + (uintptr_t)(H * W) * S;
+  // every row of words lies in the image's buffer
+  const bool safe = ((a_top + r_lo * pitch) & ~(uintptr_t)3) >= base && a_top + (r_hi - 1) * pitch + kWRow * 4 <= end;
+  for (int r0 = warp; r0 < rows; r0 += 2 * kWWarps, a += 2 * kWWarps * pitch) {
+    uint32_t w[2][4];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int r = r0 + q * kWWarps;
+      const uintptr_t aq = a + q * kWWarps * pitch, seg = aq & ~(uintptr_t)3;
+      if (r < r_lo || r >= r_hi) continue;
+      if (safe || (seg >= base && seg + kWRow * 4 <= end)) {
+        const uintptr_t p = seg + 16u * lane;  // this lane's words
+        if ((aq & 12u) == 0) {
+          const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
+          w[q][0] = v.x; w[q][1] = v.y; w[q][2] = v.z; w[q][3] = v.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) w[q][j] = __ldg(reinterpret_cast<const uint32_t *>(p) + j);
+        }
+      } else {
+        const uint4 v = edge_words(aq, base, end);
+        w[q][0] = v.x; w[q][1] = v.y; w[q][2] = v.z; w[q][3] = v.w;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int r = r0 + q * kWWarps;
+      if (r >= rows) break;
+      if (r < r_lo || r >= r_hi) {
+        *reinterpret_cast<uint4 *>(s_w + r * kWRow + lane * 4) = make_uint4(NEU, NEU, NEU, NEU);
+        continue;
+      }
+      const unsigned sh = (unsigned)((a + q * kWWarps * pitch) & 3u) * 8u;
+      if (S < 4 && sh) {
+        // the last word of lane 31 lacks its upper pixels: no output of the tile needs them (vw)
+        const uint32_t n = from_lane(w[q][0], 1);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[q][j] = __funnelshift_r(w[q][j], j < 3 ? w[q][j + 1] : n, sh);
+      }
+      if (clipped) {
+        // the lane's pixels [lo, hi) lie in the image
+        const int64_t x = x_top + (int64_t)lean * r + lane * 4 * E;
+        const int lo = (int)min(max(-x, (int64_t)0), (int64_t)4 * E), hi = (int)min(max(W - x, (int64_t)0), (int64_t)4 * E);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int l = min(max(lo - j * E, 0), E), k = min(max(hi - j * E, 0), E);  // of word j
+          const uint32_t in_m = (uint32_t)(((1ull << (8 * S * k)) - 1ull) & ~((1ull << (8 * S * l)) - 1ull));
+          w[q][j] = (w[q][j] & in_m) | (NEU & ~in_m);
+        }
+      }
+      uint4 o = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+      if (wlen > 1) {
+        RowRegs<T> m = RowRegs<T>::of(w[q]), res = m;
+        row_steps<T, SUP, 1>(m, res, wlen);
+        o = res.words();
+      }
+      *reinterpret_cast<uint4 *>(s_w + r * kWRow + lane * 4) = o;
+    }
+  }
+}
+
 template <typename T, bool SUP>
 __global__ void __launch_bounds__(kWThreads) k_window(const T *__restrict__ in, T *__restrict__ out, WindowGeom g) {
   constexpr int S = (int)sizeof(T), E = 4 / S;
   extern __shared__ __align__(16) uint32_t s_w[];  // [2 * half][kWRow]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t NEU = splat<T>(Op<T, SUP>::neutral());
   const int64_t u0 = g.u_first + (int64_t)blockIdx.x * g.vw * E;  // the tile's first pixel in its first output row
   const int64_t y0 = (int64_t)blockIdx.y * g.th;
   const int rows = g.th + 2 * g.hy, half = g.half;
   const intptr_t pitch = (intptr_t)(g.W + g.lean) * S;  // bytes from a tile row to the next
 
-  // ---- rows, two at a time per warp so that the loads of both are in flight
-  {
-    // tile rows [r_lo, r_hi) are rows of the image
-    const int r_lo = (int)max((int64_t)0, g.hy - y0), r_hi = (int)min((int64_t)rows, g.H - y0 + g.hy);
-    // first pixel of tile row 0: one word left of the tile, for the stores' shift
-    const int64_t x_top = u0 - E - g.hx - (int64_t)g.lean * g.hy;
-    const int64_t x_bot = x_top + (int64_t)g.lean * (rows - 1);
-    const uintptr_t a_top = reinterpret_cast<uintptr_t>(in) + (uintptr_t)(((y0 - g.hy) * g.W + x_top) * S);
-    uintptr_t a = a_top + warp * pitch;
-    // some row holds pixels left / right of the image
-    const bool clipped = min(x_top, x_bot) < 0 || max(x_top, x_bot) + kWRow * E > g.W;
-    const uintptr_t base = reinterpret_cast<uintptr_t>(in), end = base + (uintptr_t)(g.H * g.W) * S;
-    // every row of words lies in the image's buffer
-    const bool safe = ((a_top + r_lo * pitch) & ~(uintptr_t)3) >= base && a_top + (r_hi - 1) * pitch + kWRow * 4 <= end;
-    const int wlen = 2 * g.hx + 1;
-    for (int r0 = warp; r0 < rows; r0 += 2 * kWWarps, a += 2 * kWWarps * pitch) {
-      uint32_t w[2][4];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int r = r0 + q * kWWarps;
-        const uintptr_t aq = a + q * kWWarps * pitch, seg = aq & ~(uintptr_t)3;
-        if (r < r_lo || r >= r_hi) continue;
-        if (safe || (seg >= base && seg + kWRow * 4 <= end)) {
-          const uintptr_t p = seg + 16u * lane;  // this lane's words
-          if ((aq & 12u) == 0) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
-            w[q][0] = v.x; w[q][1] = v.y; w[q][2] = v.z; w[q][3] = v.w;
-          } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) w[q][j] = __ldg(reinterpret_cast<const uint32_t *>(p) + j);
-          }
-        } else {
-          const uint4 v = edge_words(aq, base, end);
-          w[q][0] = v.x; w[q][1] = v.y; w[q][2] = v.z; w[q][3] = v.w;
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int r = r0 + q * kWWarps;
-        if (r >= rows) break;
-        if (r < r_lo || r >= r_hi) {
-          *reinterpret_cast<uint4 *>(s_w + r * kWRow + lane * 4) = make_uint4(NEU, NEU, NEU, NEU);
-          continue;
-        }
-        const unsigned sh = (unsigned)((a + q * kWWarps * pitch) & 3u) * 8u;
-        if (S < 4 && sh) {
-          // the last word of lane 31 lacks its upper pixels: no output of the tile needs them (vw)
-          const uint32_t n = from_lane(w[q][0], 1);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) w[q][j] = __funnelshift_r(w[q][j], j < 3 ? w[q][j + 1] : n, sh);
-        }
-        if (clipped) {
-          // the lane's pixels [lo, hi) lie in the image
-          const int64_t x = x_top + (int64_t)g.lean * r + lane * 4 * E;
-          const int lo = (int)min(max(-x, (int64_t)0), (int64_t)4 * E), hi = (int)min(max(g.W - x, (int64_t)0), (int64_t)4 * E);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int l = min(max(lo - j * E, 0), E), k = min(max(hi - j * E, 0), E);  // of word j
-            const uint32_t in_m = (uint32_t)(((1ull << (8 * S * k)) - 1ull) & ~((1ull << (8 * S * l)) - 1ull));
-            w[q][j] = (w[q][j] & in_m) | (NEU & ~in_m);
-          }
-        }
-        uint4 o = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
-        if (wlen > 1) {
-          RowRegs<T> m = RowRegs<T>::of(w[q]), res = m;
-          row_steps<T, SUP, 1>(m, res, wlen);
-          o = res.words();
-        }
-        *reinterpret_cast<uint4 *>(s_w + r * kWRow + lane * 4) = o;
-      }
-    }
-  }
+  // ---- rows: from one word left of the tile, for the stores' shift
+  window_rows<T, SUP>(in, g.H, g.W, y0 - g.hy, u0 - E - g.hx - (int64_t)g.lean * g.hy, g.lean, rows, 2 * g.hx + 1, s_w);
   __syncthreads();
 
   // ---- columns: four warps side by side, two groups of rows
@@ -311,9 +353,7 @@ __global__ void __launch_bounds__(kWThreads) k_window(const T *__restrict__ in, 
   const int c = (warp & 3) * 31 + lane - 1;  // lane 0 only lends its word to lane 1
   const int gh = g.th / 2, ya = (warp >> 2) * gh;
   const int yb = (int)min((int64_t)(ya + gh), g.H - y0);
-  const int64_t x_end = u0 + (int64_t)g.lean * (g.th - 1);
-  const bool inner = min(u0, x_end) >= E && max(u0, x_end) + g.vw * E <= g.W;
-  const bool mine = lane > 0 && c < g.vw;
+  const TileStore<T> st(g.W, u0, g.lean, g.th, g.vw, c);
   const uint32_t *q = s_w + c + 1 + ya * kWRow;
   uintptr_t a = reinterpret_cast<uintptr_t>(out) + (uintptr_t)(((y0 + ya) * g.W + u0 + (int64_t)g.lean * ya) * S);
   constexpr int U = 4;
@@ -336,24 +376,7 @@ __global__ void __launch_bounds__(kWThreads) k_window(const T *__restrict__ in, 
 #pragma unroll
     for (int k = 0; k < U; ++k) {
       if (y + k >= yb) break;  // uniform
-      const uintptr_t ak = a + k * pitch;
-      const unsigned mis = S < 4 ? (unsigned)(ak & 3u) : 0u;  // bytes past an aligned word
-      uint32_t o = v[k].word();
-      if (mis) o = __funnelshift_l(__shfl_up_sync(0xffffffffu, o, 1), o, mis * 8u);
-      if (!mine) continue;
-      T *dst = reinterpret_cast<T *>((ak & ~(uintptr_t)3) + 4 * (intptr_t)c);
-      if (inner) {
-        *reinterpret_cast<uint32_t *>(dst) = o;
-      } else {
-        const int64_t x = u0 + (int64_t)g.lean * (y + k) + c * E - (int)mis / S;  // the word's first pixel
-        if (x >= 0 && x + E <= g.W) {
-          *reinterpret_cast<uint32_t *>(dst) = o;
-        } else if (S < 4 && x + E > 0 && x < g.W) {
-#pragma unroll
-          for (int e = 0; e < E; ++e)
-            if (x + e >= 0 && x + e < g.W) dst[e] = (T)(o >> (8 * S * e));
-        }
-      }
+      st.put(a + k * pitch, y + k, v[k].word());
     }
   }
 }
@@ -390,6 +413,154 @@ pg_status window_t(const pg_image &in, const pg_image &out, WindowGeom g, cudaSt
   return cuda_status(cudaGetLastError(), "window kernel launch");
 }
 
+// ------------------------------------------------------------------ neighbour lists
+// Erosion / dilation by an offset list (ero_dil_runtime_nl_se_t.hpp:129-193, clipped; like the gather kernel
+// the extremum always holds the neutral value).  The list is cut into chords, runs of offsets along a row; the
+// chords of one length, first column and slice form a group, whose row windows are formed once and serve
+// all its rows: a disk of radius 7 has 149 offsets, 15 chords and 5 groups.  Per group the tile's rows go to
+// shared memory as windows of the chord's length, moved by its first column (the loads take any alignment),
+// and every thread adds the chords' rows to its R outputs, kept in registers.
+// Bound: the ALU pipe, 4-5 instructions per chord and word of outputs plus a row pass per group.  2048^2 u8,
+// radius 7: 905 us (149 bounds-checked loads per pixel, small_se.cu) -> 29 us; radius 2 f32 121 -> 25 us.
+struct ChordGroup {
+  int x0;                  // first column of the chords
+  short dz, len;           // slice, pixels
+  short dy_min, dy_max;    // rows
+  short first, count;      // in ChordTable::dy
+};
+constexpr int kMaxGroups = 64, kMaxChords = 512, kMaxSpan = 96;
+struct ChordTable {
+  int n;
+  ChordGroup g[kMaxGroups];
+  short dy[kMaxChords];
+};
+
+template <typename T, bool SUP, int R>
+__global__ void __launch_bounds__(kWThreads, sizeof(T) == 1 ? 3 : 4) k_chords(const T *__restrict__ in, T *__restrict__ out, int64_t D, int64_t H,
+                                                      int64_t W, int vw, const __grid_constant__ ChordTable t) {
+  constexpr int S = (int)sizeof(T), E = 4 / S, TH = 2 * R;
+  extern __shared__ __align__(16) uint32_t s_w[];  // [TH + span of dy][kWRow]
+  using A = Acc<T, SUP>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t u0 = (int64_t)blockIdx.x * vw * E, y0 = (int64_t)blockIdx.y * TH, z = blockIdx.z;
+  const int c = (warp & 3) * 31 + lane - 1, ya = (warp >> 2) * R;  // as in k_window
+  A acc[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) acc[i] = A::of(splat<T>(Op<T, SUP>::neutral()));
+  for (int k = 0; k < t.n; ++k) {
+    const ChordGroup &g = t.g[k];
+    if (z + g.dz < 0 || z + g.dz >= D) continue;  // uniform
+    __syncthreads();                              // the last group's windows have been read
+    window_rows<T, SUP>(in + (z + g.dz) * H * W, H, W, y0 + g.dy_min, u0 - E + g.x0, 0, TH + g.dy_max - g.dy_min, g.len, s_w);
+    __syncthreads();
+    const uint32_t *q = s_w + c + 1 + (ya - g.dy_min) * kWRow;
+    int j = g.first;
+    const int end = g.first + g.count;
+    for (; j + 1 < end; j += 2) {  // two chords at a time: one instruction takes both
+      const uint32_t *p0 = q + t.dy[j] * kWRow, *p1 = q + t.dy[j + 1] * kWRow;
+#pragma unroll
+      for (int i = 0; i < R; ++i) acc[i] = acc[i].with(A::of(p0[i * kWRow])).with(A::of(p1[i * kWRow]));
+    }
+    if (j < end) {
+      const uint32_t *p0 = q + t.dy[j] * kWRow;
+#pragma unroll
+      for (int i = 0; i < R; ++i) acc[i] = acc[i].with(A::of(p0[i * kWRow]));
+    }
+  }
+  const TileStore<T> st(W, u0, 0, TH, vw, c);
+  const intptr_t pitch = (intptr_t)W * S;
+  const uintptr_t a = reinterpret_cast<uintptr_t>(out) + (uintptr_t)(((z * H + y0 + ya) * W + u0) * S);
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    if (y0 + ya + i >= H) break;  // uniform
+    st.put(a + i * pitch, ya + i, acc[i].word());
+  }
+}
+
+template <typename T, bool SUP, int R>
+pg_status chords_r(const pg_image &in, const pg_image &out, const ChordTable &t, int vw, int tiles_x, int span,
+                   cudaStream_t s) {
+  const Dims d = dims_of(in);
+  static std::atomic<uint64_t> attr_devices{0};
+  int dev = 0;
+  PG_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
+  const uint64_t bit = 1ull << (dev & 63);
+  if (!(attr_devices.load() & bit)) {
+    PG_CUDA_TRY(cudaFuncSetAttribute(k_chords<T, SUP, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWSmemMax),
+                "neighbour-list kernel smem attribute");
+    attr_devices.fetch_or(bit);
+  }
+  const dim3 grid((unsigned)tiles_x, (unsigned)ceil_div(d.ny, 2 * R), (unsigned)d.nz);
+  k_chords<T, SUP, R><<<grid, kWThreads, (size_t)(2 * R + span) * kWRow * 4, s>>>(
+      static_cast<const T *>(in.data), static_cast<T *>(out.data), d.nz, d.ny, d.nx, vw, t);
+  return cuda_status(cudaGetLastError(), "neighbour-list kernel launch");
+}
+
+template <typename T, bool SUP>
+pg_status chords_t(const pg_image &in, const pg_image &out, const ChordTable &t, int max_len, int span, cudaStream_t s) {
+  constexpr int E = 4 / (int)sizeof(T);
+  const Dims d = dims_of(in);
+  const int vw = std::min((kWRow * E - (max_len - 1)) / E - 2, kWOut) & ~7;  // as in window_t
+  const bool mis = E > 1 && (d.nx % E != 0 || reinterpret_cast<uintptr_t>(out.data) % 4 != 0);
+  const int tiles_x = (int)ceil_div(d.nx + (mis ? E - 1 : 0), (int64_t)vw * E);
+  // Rows a thread holds, half a tile's: what three (u8, two registers a row) or four CTAs per SM leave room for
+  // (2048^2 u8, radius 5: 12 rows 29 us, 16 rows 35, 8 rows 34; f32: 16 rows 49, 12 rows 51, 8 rows 60); 4
+  // where the image would not give every SM a tile.
+  constexpr int R = sizeof(T) == 1 ? 12 : 16;
+  if (tiles_x * ceil_div(d.ny, 2 * R) * d.nz < num_sms()) return chords_r<T, SUP, 4>(in, out, t, vw, tiles_x, span, s);
+  return chords_r<T, SUP, R>(in, out, t, vw, tiles_x, span, s);
+}
+
+// The list as chords; false where it has too many, or where they are so short that gathering the offsets one
+// by one costs less (per 32-bit word of outputs: 14 instructions per offset and pixel, against 50 per group and
+// 5 per chord).
+bool make_chords(const int32_t *offsets, int n, int rank, int pixels_per_word, int max_len, ChordTable &t, int &span,
+                 int &longest) {
+  // offsets and chords as one sortable word each (fields below 2^15, biased): dz, dy, dx and dz, x0, len, dy
+  constexpr int kFar = 16383, kBias = 16384;
+  uint64_t key[4096], chord[kMaxChords];
+  if (n > 4096) return false;
+  for (int k = 0; k < n; ++k) {
+    uint64_t v = 0;
+    for (int r = 0; r < 3; ++r) {
+      const int o = r < 3 - rank ? 0 : offsets[k * rank + r - (3 - rank)];
+      if (o < -kFar || o > kFar) return false;
+      v = (v << 16) | (uint64_t)(o + kBias);
+    }
+    key[k] = v;
+  }
+  std::sort(key, key + n);
+  n = (int)(std::unique(key, key + n) - key);
+  int nc = 0;
+  for (int i = 0, j; i < n; i = j) {
+    // a run of a row: consecutive words (a column's neighbour never reaches the next field)
+    for (j = i + 1; j < n && key[j] == key[j - 1] + 1 && j - i < max_len;) ++j;
+    if (nc == kMaxChords) return false;
+    const uint64_t dz = key[i] >> 32, dy = (key[i] >> 16) & 0xffff, dx = key[i] & 0xffff;
+    chord[nc++] = (dz << 48) | (dx << 32) | ((uint64_t)(j - i) << 16) | dy;
+  }
+  std::sort(chord, chord + nc);
+  auto row = [&](int i) { return (int)(chord[i] & 0xffff) - kBias; };
+  t.n = 0;
+  span = 0;
+  longest = 1;
+  for (int i = 0, j; i < nc; i = j) {
+    if (t.n == kMaxGroups) return false;
+    ChordGroup &g = t.g[t.n++];
+    for (j = i; j < nc && (chord[j] >> 16) == (chord[i] >> 16) && row(j) - row(i) <= kMaxSpan; ++j) t.dy[j] = (short)row(j);
+    g.dz = (short)((int)(chord[i] >> 48) - kBias);
+    g.x0 = (int)((chord[i] >> 32) & 0xffff) - kBias;
+    g.len = (short)((chord[i] >> 16) & 0xffff);
+    g.dy_min = (short)row(i);
+    g.dy_max = (short)row(j - 1);
+    g.first = (short)i;
+    g.count = (short)(j - i);
+    span = std::max(span, (int)g.dy_max - g.dy_min);
+    longest = std::max(longest, (int)g.len);
+  }
+  return 50 * t.n + 5 * nc <= 14 * n * pixels_per_word;
+}
+
 }  // namespace
 
 bool window_ok(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, int lean) {
@@ -419,6 +590,26 @@ bool try_window(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx,
     case PG_PTYPE_U16: *st = dilate ? window_t<uint16_t, true>(in, out, g, s) : window_t<uint16_t, false>(in, out, g, s); return true;
     case PG_PTYPE_I32: *st = dilate ? window_t<int32_t, true>(in, out, g, s) : window_t<int32_t, false>(in, out, g, s); return true;
     case PG_PTYPE_F32: *st = dilate ? window_t<float, true>(in, out, g, s) : window_t<float, false>(in, out, g, s); return true;
+    default: return false;
+  }
+}
+
+bool try_chords(const pg_image &in, const pg_image &out, const int32_t *offsets, int n, bool dilate, cudaStream_t s,
+                pg_status *st) {
+  const int es = elem_size(in.ptype);
+  if (in.rank < 2 || (es != 1 && es != 2 && es != 4)) return false;
+  const Dims d = dims_of(in);
+  if (d.ny < 16 || d.nx < 1 || d.ny > (1 << 18) || d.nx > (1 << 30) || d.nz > 65535) return false;
+  const uintptr_t pixel = (uintptr_t)es - 1;
+  if ((reinterpret_cast<uintptr_t>(in.data) | reinterpret_cast<uintptr_t>(out.data)) & pixel) return false;
+  ChordTable t;
+  int span = 0, longest = 1;
+  if (!make_chords(offsets, n, in.rank, 4 / es, es == 4 ? 32 : 64, t, span, longest)) return false;
+  switch (in.ptype) {
+    case PG_PTYPE_U8: *st = dilate ? chords_t<uint8_t, true>(in, out, t, longest, span, s) : chords_t<uint8_t, false>(in, out, t, longest, span, s); return true;
+    case PG_PTYPE_U16: *st = dilate ? chords_t<uint16_t, true>(in, out, t, longest, span, s) : chords_t<uint16_t, false>(in, out, t, longest, span, s); return true;
+    case PG_PTYPE_I32: *st = dilate ? chords_t<int32_t, true>(in, out, t, longest, span, s) : chords_t<int32_t, false>(in, out, t, longest, span, s); return true;
+    case PG_PTYPE_F32: *st = dilate ? chords_t<float, true>(in, out, t, longest, span, s) : chords_t<float, false>(in, out, t, longest, span, s); return true;
     default: return false;
   }
 }
