@@ -181,6 +181,24 @@ struct Scratch {
   template <typename U> U *as() const { return static_cast<U *>(ptr); }
 };
 
+// One 8-byte word of pinned host memory that kernels write and the host reads after synchronising their
+// stream (status.cu): a result comes back without a copy call.  The words are a fixed set of kHostSlots per
+// process, shared by all threads; `word` is null while all of them are taken (or none could be made), and the
+// caller then copies from device memory.
+constexpr int kHostSlots = 64;
+class HostSlot {
+ public:
+  HostSlot();
+  ~HostSlot();
+  HostSlot(const HostSlot &) = delete;
+  HostSlot &operator=(const HostSlot &) = delete;
+  long long *word = nullptr;  // device-visible; the host reads it through value()
+  long long value() const;
+
+ private:
+  int index_ = -1;
+};
+
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // The value of a pg_scalar as pixel type T.  The entry points check that the scalar holds T's own
@@ -254,6 +272,15 @@ inline bool rows_aligned(const pg_image &in, const pg_image &out, int unit) {
          (reinterpret_cast<uintptr_t>(in.data) | reinterpret_cast<uintptr_t>(out.data)) % (uintptr_t)unit == 0;
 }
 
+// Device status words (0: none), one per file whose kernels can give up; pg_check_device reads them all.
+cudaError_t recon_status_word(void **p);
+cudaError_t rect_status_word(void **p);
+cudaError_t diag_status_word(void **p);
+cudaError_t oct_status_word(void **p);
+cudaError_t small_tile_status_word(void **p);
+cudaError_t open_status_word(void **p);
+cudaError_t label_status_word(void **p);
+
 // ------------------------------------------------------------------ kernel entry points
 // (host launchers, implemented in the .cu files)
 pg_status launch_small_se(const pg_image &in, const pg_image &out, int se, bool dilate, cudaStream_t s);
@@ -272,17 +299,14 @@ bool try_segment_open(const pg_image &in, const pg_image &out, int dy, int dx, i
                       pg_status *st);
 bool try_segment_gradient(const pg_image &in, const pg_image &out, int dy, int dx, int k, cudaStream_t s,
                           pg_status *st);  // dilation - erosion by that segment in one pass
-int take_diag_status();  // device status of the diagonal tile kernel since the last call (0: none)
 // The octagon's n = n_cross + n_square passes in one shared-memory tile kernel (octagon.cu): u8 images
 // for 5 <= n <= 16, u16 for 3 <= n <= 16, rows of a multiple of 16 bytes.  n_square = 0: the cross
 // iterated n times (SECross2D, iter = n).
 bool try_octagon_tile(const pg_image &in, const pg_image &out, int n_cross, int n_square, bool dilate, cudaStream_t s,
                       pg_status *st);
-int take_oct_status();  // device status of the octagon tile kernel since the last call (0: none)
 // 3x3 square / cross and 3-pixel X / Y segments on TMA tiles (small_tile.cu): 2D u8 / u16 images with
 // rows of a multiple of 16 bytes.
 bool try_small_tile(const pg_image &in, const pg_image &out, int se, bool dilate, cudaStream_t s, pg_status *st);
-int take_small_tile_status();  // device status of the small-SE tile kernel since the last call (0: none)
 // Boxes and vertical / 45- / 135-degree segments (lean = the pixels a row moves right per row: hx = 0) of any
 // half lengths up to 63 (row windows of at most half a tile row), any row length and alignment (window.cu):
 // 1-, 2- and 4-byte pixels, images of at least 16 rows.
@@ -303,11 +327,8 @@ bool try_rect_gradient(const pg_image &in, const pg_image &out, int64_t hy, int6
 // One-pass opening / closing by an X segment (rect_open.cu): hy = 0, hx = 7, 15, 31.
 bool try_rect_open(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, bool opening, cudaStream_t s,
                    pg_status *st);
-int take_open_status();  // device status of the one-pass opening kernel since the last call (0: none)
 // connected-component labelling into an int64 image (label.cu); count may be null
 pg_status launch_label(const pg_image &in, int se, const pg_image &out, bool flat, int64_t *count, cudaStream_t s);
-int take_label_status();
-int take_rect_status();  // device status of the fused square kernel since the last call (0: none)
 pg_status launch_copy(const pg_image &in, const pg_image &out, cudaStream_t s);
 pg_status launch_sub(const pg_image &a, const pg_image &b, const pg_image &out, cudaStream_t s);
 pg_status launch_sat_const(const pg_image &in, const pg_scalar &v, bool add, const pg_image &out, cudaStream_t s);

@@ -508,11 +508,6 @@ bool try_segment_gradient(const pg_image &in, const pg_image &out, int dy, int d
   return segment_try<4>(in, out, dy, dx, k, s, st);
 }
 
-int take_diag_status() {
-  int st = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&st, g_diag_status, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  if (st != 0 && cudaMemcpyToSymbol(g_diag_status, &zero, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  return st;
-}
+cudaError_t diag_status_word(void **p) { return cudaGetSymbolAddress(p, g_diag_status); }
 
 }  // namespace pg

@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(kLThreads) k_label_flatten(int32_t *par, unsig
 // counts.  A root's parent word becomes -1 - number (numbers start at 1; -1 stays the background).
 __global__ void __launch_bounds__(kLThreads) k_label_number(int32_t *__restrict__ par, const unsigned *__restrict__ roots,
                                                             const int32_t *__restrict__ cnt, LabelGeom g, int64_t words,
-                                                            int log_seg, int64_t *__restrict__ total) {
+                                                            int log_seg, long long *__restrict__ total) {
   __shared__ int32_t s_w[2][kLThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int32_t before = 0;
@@ -457,7 +457,10 @@ __global__ void __launch_bounds__(kLThreads) k_label_number(int32_t *__restrict_
   int32_t base = 0;
 #pragma unroll
   for (int w = 0; w < kLThreads / 32; ++w) base += s_w[0][w];
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = (int64_t)base + cnt[blockIdx.x];
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    *(volatile long long *)total = (long long)base + cnt[blockIdx.x];
+    __threadfence_system();  // it may be host memory
+  }
   if (cnt[blockIdx.x] == 0) return;
   const int64_t end = min(words, ((int64_t)blockIdx.x + 1) << log_seg);
   int buf = 1;
@@ -562,7 +565,9 @@ pg_status label_t(const pg_image &in, const pg_image &out, unsigned edges, int64
   int32_t *par = work.as<int32_t>();
   unsigned *roots = reinterpret_cast<unsigned *>(work.as<char>() + par_bytes);
   int32_t *cnt = reinterpret_cast<int32_t *>(work.as<char>() + par_bytes + root_bytes);
-  int64_t *total = reinterpret_cast<int64_t *>(cnt + kLSegments);
+  HostSlot slot;  // the count goes straight to the host, where one waits for it
+  long long *device_total = reinterpret_cast<long long *>(cnt + kLSegments);
+  long long *total = count && slot.word ? slot.word : device_total;
   int64_t *o = static_cast<int64_t *>(out.data);
   const T *src = static_cast<const T *>(in.data);
   PG_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)nseg, s), "clear label counts");
@@ -581,8 +586,10 @@ pg_status label_t(const pg_image &in, const pg_image &out, unsigned edges, int64
   else k_label_resolve<false><<<rg, kLThreads, 0, s>>>(par, n, o);
   PG_TRY(cuda_status(cudaGetLastError(), "labelling kernels launch"));
   if (count) {
-    PG_CUDA_TRY(cudaMemcpyAsync(count, total, sizeof(int64_t), cudaMemcpyDeviceToHost, s), "label count copy");
+    if (total == device_total)
+      PG_CUDA_TRY(cudaMemcpyAsync(count, total, sizeof(int64_t), cudaMemcpyDeviceToHost, s), "label count copy");
     PG_CUDA_TRY(cudaStreamSynchronize(s), "label count synchronisation");
+    if (total != device_total) *count = slot.value();
   }
   return PG_OK;
 }
@@ -609,11 +616,6 @@ pg_status launch_label(const pg_image &in, int se, const pg_image &out, bool fla
   return PG_OK;
 }
 
-int take_label_status() {
-  int st = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&st, g_label_status, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  if (st != 0 && cudaMemcpyToSymbol(g_label_status, &zero, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  return st;
-}
+cudaError_t label_status_word(void **p) { return cudaGetSymbolAddress(p, g_label_status); }
 
 }  // namespace pg

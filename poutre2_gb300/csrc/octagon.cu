@@ -191,11 +191,6 @@ bool try_octagon_tile(const pg_image &in, const pg_image &out, int n_cross, int 
   return true;
 }
 
-int take_oct_status() {
-  int st = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&st, g_oct_status, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  if (st != 0 && cudaMemcpyToSymbol(g_oct_status, &zero, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  return st;
-}
+cudaError_t oct_status_word(void **p) { return cudaGetSymbolAddress(p, g_oct_status); }
 
 }  // namespace pg

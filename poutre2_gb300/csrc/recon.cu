@@ -1529,6 +1529,8 @@ void destroy_batch_plan(pg_batch_plan *p) {
   delete p;
 }
 
+cudaError_t recon_status_word(void **p) { return cudaGetSymbolAddress(p, g_recon_status); }
+
 // ------------------------------------------------------------------ allocation-free variant
 // For callers that must not touch the device allocator (see pg_reconstruction_noalloc in
 // include/poutre_gb300.h).  Its only scratch -- the control block and the tile worklist --
@@ -1640,31 +1642,6 @@ static pg_status reconstruction_noalloc(bool dilate, bool conn8, const pg_image 
 }  // namespace pg
 
 extern "C" {
-
-// Synchronises `stream`, then reads and clears the device status of the reconstruction
-// kernels (PG_ERR_NOT_CONVERGED if one gave up since the last check).
-pg_status pg_check_device(pg_stream_t stream) {
-  PG_CUDA_TRY(cudaStreamSynchronize(reinterpret_cast<cudaStream_t>(stream)), "stream synchronisation");
-  int st = 0, zero = 0;
-  PG_CUDA_TRY(cudaMemcpyFromSymbol(&st, pg::g_recon_status, sizeof(int)), "read device status");
-  if (st != 0) {
-    PG_CUDA_TRY(cudaMemcpyToSymbol(pg::g_recon_status, &zero, sizeof(int)), "clear device status");
-    return pg::fail(static_cast<pg_status>(st), "reconstruction did not converge within its round cap or wait limit");
-  }
-  if (const int rs = pg::take_rect_status())
-    return pg::fail(static_cast<pg_status>(rs), "a box tile load did not complete within its wait limit");
-  if (const int ds = pg::take_diag_status())
-    return pg::fail(static_cast<pg_status>(ds), "a segment tile load did not complete within its wait limit");
-  if (const int os8 = pg::take_oct_status())
-    return pg::fail(static_cast<pg_status>(os8), "an octagon tile load did not complete within its wait limit");
-  if (const int ss = pg::take_small_tile_status())
-    return pg::fail(static_cast<pg_status>(ss), "a small-SE tile load did not complete within its wait limit");
-  if (const int os = pg::take_open_status())
-    return pg::fail(static_cast<pg_status>(os), "an opening tile load did not complete within its wait limit");
-  if (const int ls = pg::take_label_status())
-    return pg::fail(static_cast<pg_status>(ls), "a labelling union-find loop exceeded its iteration limit");
-  return PG_OK;
-}
 
 // Test hooks: lower the reconstruction's round / visit cap and its device wait limit so that a test
 // can make a bounded wait run out and read PG_ERR_NOT_CONVERGED back; 0 restores the defaults.

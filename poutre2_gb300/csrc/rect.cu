@@ -263,11 +263,6 @@ bool try_rect_gradient(const pg_image &in, const pg_image &out, int64_t hy, int6
   }
 }
 
-int take_rect_status() {
-  int st = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&st, g_rect_status, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  if (st != 0 && cudaMemcpyToSymbol(g_rect_status, &zero, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  return st;
-}
+cudaError_t rect_status_word(void **p) { return cudaGetSymbolAddress(p, g_rect_status); }
 
 }  // namespace pg

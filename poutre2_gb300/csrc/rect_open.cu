@@ -205,11 +205,6 @@ bool try_rect_open(const pg_image &in, const pg_image &out, int64_t hy, int64_t 
   }
 }
 
-int take_open_status() {
-  int st = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&st, g_open_status, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  if (st != 0 && cudaMemcpyToSymbol(g_open_status, &zero, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  return st;
-}
+cudaError_t open_status_word(void **p) { return cudaGetSymbolAddress(p, g_open_status); }
 
 }  // namespace pg

@@ -417,11 +417,6 @@ bool try_small_tile(const pg_image &in, const pg_image &out, int se, bool dilate
   return true;
 }
 
-int take_small_tile_status() {
-  int st = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&st, g_small_tile_status, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  if (st != 0 && cudaMemcpyToSymbol(g_small_tile_status, &zero, sizeof(int)) != cudaSuccess) return (int)PG_ERR_CUDA;
-  return st;
-}
+cudaError_t small_tile_status_word(void **p) { return cudaGetSymbolAddress(p, g_small_tile_status); }
 
 }  // namespace pg
