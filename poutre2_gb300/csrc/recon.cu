@@ -37,6 +37,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "words.cuh"
 
 namespace pg {
 
@@ -375,97 +376,110 @@ __device__ void process_tile(const RImg &im, const RParams<T> &P, int t_local, i
   __syncthreads();
 }
 
+// The image that holds a tile, and the tile's index in it.  `begin`: the images' first tiles in shared memory,
+// or null (the search then reads the device table, a dependent load per step).
 template <typename T>
-__device__ __forceinline__ const RImg &image_of(const RParams<T> &P, int tile, int &t_local) {
+__device__ __forceinline__ const RImg &image_of(const RParams<T> &P, int tile, int &t_local, const int *begin = nullptr) {
   if (P.nimg == 1) { t_local = tile; return P.single; }
   int lo = 0, hi = P.nimg - 1;
   while (lo < hi) {  // last image whose tile_begin <= tile
     const int mid = (lo + hi + 1) >> 1;
-    if (P.imgs[mid].tile_begin <= tile) lo = mid; else hi = mid - 1;
+    if ((begin ? begin[mid] : P.imgs[mid].tile_begin) <= tile) lo = mid; else hi = mid - 1;
   }
-  t_local = tile - P.imgs[lo].tile_begin;
+  t_local = tile - (begin ? begin[lo] : P.imgs[lo].tile_begin);
   return P.imgs[lo];
 }
 
-// Epilogue over every pixel of every image, after the last round: the binary h-maxima
-// comparison or the leveling clip by the reference.  Pure streaming: 16-byte vectors when the
-// image's buffers allow it, otherwise EPI_UNROLL independent elements per thread per step, so
-// that many loads are in flight (a plain grid-stride loop over single pixels would wait for
-// each load in turn).
+// The pixels of every image cut into as many runs as it has tiles, one warp per run (the images of a batch
+// go side by side; image after image over the whole grid, each waited for its loads in turn: 0.9 of the
+// 6.2 ms of a 512-image batch, twice): calls run(image, first pixel, end), runs on 16-pixel boundaries.
+template <typename T, typename F>
+__device__ __forceinline__ void for_pixel_runs(const RParams<T> &P, const int *begin, F run) {
+  const int warps = (int)((gridDim.x * blockDim.x) >> 5);
+  for (int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); t < P.ntiles; t += warps) {
+    int c = 0;
+    const RImg &im = image_of(P, t, c, begin);
+    const int64_t n = im.H * im.W, tiles = (int64_t)im.tiles_x * im.tiles_y;
+    const int64_t len = ((n + tiles - 1) / tiles + 15) / 16 * 16, lo = c * len;
+    if (lo < n) run(im, lo, min(lo + len, n));
+  }
+}
+
+// Epilogue of pixels [lo, hi) of an image, by one warp, after the last round: the binary h-maxima comparison or
+// the leveling clip by the reference.  Pure streaming: 16-byte vectors when the image's buffers allow it,
+// otherwise EPI_UNROLL independent elements per lane per step, so that many loads are in flight.
 static constexpr int EPI_UNROLL = 8;
 
 template <typename T, bool SUP>
 __device__ __forceinline__ uint8_t epi_binary(T ref, T rec) { return ref > rec ? 255 : 0; }
 
 template <typename T, bool SUP>
-__device__ void epilogue_image(const RImg &im, int epi, int64_t tid, int64_t nth) {
-  const int64_t n = im.H * im.W;
+__device__ __forceinline__ void epilogue_run(const RImg &im, int epi, int64_t lo, int64_t hi) {
+  const int lane = threadIdx.x & 31;
   const T *rec = static_cast<const T *>(im.rec);
   const T *ref = static_cast<const T *>(im.mask);
   constexpr int VE = 16 / (int)sizeof(T);  // pixels per 16-byte vector
   const bool vec = ((reinterpret_cast<uintptr_t>(rec) | reinterpret_cast<uintptr_t>(ref) |
                      reinterpret_cast<uintptr_t>(im.out)) % 16 == 0);
-  int64_t done = 0;
+  int64_t done = lo;
   if (epi == EPI_BINARY_SUP) {
     uint8_t *o = static_cast<uint8_t *>(im.out);
     if (vec && sizeof(T) == 1) {
-      // 16 u8 pixels per thread and step: byte-wise unsigned compare gives 0xff / 0x00 directly
-      const int64_t nv = n / 16;
-      for (int64_t j = tid; j < nv; j += nth) {
+      // 16 u8 pixels per lane and step: byte-wise unsigned compare gives 0xff / 0x00 directly
+#pragma unroll 2
+      for (int64_t j = lo / 16 + lane; j < hi / 16; j += 32) {
         const uint4 a = __ldg(reinterpret_cast<const uint4 *>(ref) + j);
         const uint4 b = __ldcg(reinterpret_cast<const uint4 *>(rec) + j);
         reinterpret_cast<uint4 *>(o)[j] =
             make_uint4(__vcmpgtu4(a.x, b.x), __vcmpgtu4(a.y, b.y), __vcmpgtu4(a.z, b.z), __vcmpgtu4(a.w, b.w));
       }
-      done = nv * 16;
+      done = hi / 16 * 16;
     }
-    for (int64_t i0 = done + tid; i0 < n; i0 += nth * EPI_UNROLL) {
+    for (int64_t i0 = done + lane; i0 < hi; i0 += 32 * EPI_UNROLL) {
       T a[EPI_UNROLL], b[EPI_UNROLL];
 #pragma unroll
       for (int u = 0; u < EPI_UNROLL; ++u) {
-        const int64_t i = i0 + u * nth;
-        a[u] = i < n ? ldg(ref + i) : T(0);
-        b[u] = i < n ? ld_cg(rec + i) : T(0);
+        const int64_t i = i0 + u * 32;
+        a[u] = i < hi ? ldg(ref + i) : T(0);
+        b[u] = i < hi ? ld_cg(rec + i) : T(0);
       }
 #pragma unroll
       for (int u = 0; u < EPI_UNROLL; ++u) {
-        const int64_t i = i0 + u * nth;
-        if (i < n) o[i] = epi_binary<T, SUP>(a[u], b[u]);
+        const int64_t i = i0 + u * 32;
+        if (i < hi) o[i] = epi_binary<T, SUP>(a[u], b[u]);
       }
     }
   } else {  // EPI_CLIP_REF: low leveling min(rec, ref), high leveling max(rec, ref)
     T *o = static_cast<T *>(im.out);
     if (vec) {
-      const int64_t nv = n / VE;
-      for (int64_t j = tid; j < nv; j += nth) {
+#pragma unroll 2
+      for (int64_t j = lo / VE + lane; j < hi / VE; j += 32) {
         const Pack<T> a = Pack<T>::load_cg(rec + j * VE);
         const Pack<T> b = Pack<T>::load(ref + j * VE);
         Pack<T>::template op<!SUP>(a, b).store(o + j * VE);
       }
-      done = nv * VE;
+      done = hi / VE * VE;
     }
-    for (int64_t i0 = done + tid; i0 < n; i0 += nth * EPI_UNROLL) {
+    for (int64_t i0 = done + lane; i0 < hi; i0 += 32 * EPI_UNROLL) {
       T a[EPI_UNROLL], b[EPI_UNROLL];
 #pragma unroll
       for (int u = 0; u < EPI_UNROLL; ++u) {
-        const int64_t i = i0 + u * nth;
-        a[u] = i < n ? ld_cg(rec + i) : T(0);
-        b[u] = i < n ? ldg(ref + i) : T(0);
+        const int64_t i = i0 + u * 32;
+        a[u] = i < hi ? ld_cg(rec + i) : T(0);
+        b[u] = i < hi ? ldg(ref + i) : T(0);
       }
 #pragma unroll
       for (int u = 0; u < EPI_UNROLL; ++u) {
-        const int64_t i = i0 + u * nth;
-        if (i < n) o[i] = Op<T, !SUP>::apply(a[u], b[u]);
+        const int64_t i = i0 + u * 32;
+        if (i < hi) o[i] = Op<T, !SUP>::apply(a[u], b[u]);
       }
     }
   }
 }
 
 template <typename T, bool SUP>
-__device__ void recon_epilogue(const RParams<T> &P) {
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nth = (int64_t)gridDim.x * blockDim.x;
-  for (int k = 0; k < P.nimg; ++k) epilogue_image<T, SUP>((P.nimg == 1) ? P.single : P.imgs[k], P.epi, tid, nth);
+__device__ void recon_epilogue(const RParams<T> &P, const int *begin) {
+  for_pixel_runs(P, begin, [&](const RImg &im, int64_t lo, int64_t hi) { epilogue_run<T, SUP>(im, P.epi, lo, hi); });
 }
 
 template <typename T, bool SUP, bool CONN8, int RT = tile_side<T>()>
@@ -516,7 +530,7 @@ __global__ void __launch_bounds__(RT) k_reconstruct(RParams<T> P) {
     g_recon_rounds = round;
   }
   if (!ok || P.epi == EPI_NONE) return;
-  recon_epilogue<T, SUP>(P);
+  recon_epilogue<T, SUP>(P, nullptr);
 }
 
 // ------------------------------------------------------------------ register tiles
@@ -535,12 +549,11 @@ __global__ void __launch_bounds__(RT) k_reconstruct(RParams<T> P) {
 static constexpr int kRegWarps = 4;
 static constexpr int kRP = 33;  // pitch in words of the per-warp shared arrays
 
-template <typename T> using RegS = std::conditional_t<(sizeof(T) < 4), uint32_t, T>;
 
 // Mask reads inside the sweeps: a volatile shared load is performed where it is written, so the
 // compiler does not keep the whole 32x32 mask in registers across sweeps (which would cost 64
 // registers per thread and most of the occupancy).
-template <typename T> __device__ __forceinline__ T lds_mask(const RegS<T> *p) {
+template <typename T> __device__ __forceinline__ T lds_mask(const T *p) {
   const unsigned addr = (unsigned)__cvta_generic_to_shared(p);
   uint32_t r;
   asm volatile("ld.volatile.shared.b32 %0, [%1];" : "=r"(r) : "r"(addr));
@@ -557,21 +570,11 @@ template <typename T> __device__ __forceinline__ T shfl_dn1(T v) {
   else return __shfl_down_sync(0xffffffffu, v, 1);
 }
 
-// element e (a compile-time constant after unrolling) of a 16-byte vector of 1- or 2-byte pixels
-template <typename T> __device__ __forceinline__ T vec_elem(const uint4 &v, int e) {
-  constexpr int PW = 4 / (int)sizeof(T);  // pixels per 32-bit word
-  const int w = e / PW, sh = (e % PW) * 8 * (int)sizeof(T);
-  const uint32_t word = w == 0 ? v.x : w == 1 ? v.y : w == 2 ? v.z : v.w;
-  return (T)(word >> sh);
-}
-
-// Sweep sets of a 32x32 tile of 1- or 2-byte pixels with two rows per 32-bit register: pair p
-// holds row p (low half) and row 31 - p (high half) of the lane's column, so the two chains that
-// the vertical sweeps run at once (down over the top half with up over the bottom half, then the
-// reverse) advance together in one 2x16-bit min/max per step; after the transpose, pair c holds
-// columns c and 31 - c of the lane's row and the horizontal chains pair up the same way.  The
-// masks are packed the same way.  Same updates, in the same order, as the
-// unpacked sweeps.  Returns through v (unpacked) and the flags; s_m is overwritten.
+// Tiles of 1- or 2-byte pixels hold two rows per 32-bit register: pair p holds row p (low half) and row 31 - p
+// (high half) of the lane's column, so the two chains that the vertical sweeps run at once (down over the top
+// half with up over the bottom half, then the reverse) advance together in one 2x16-bit min/max per step;
+// after the transpose, pair c holds columns c and 31 - c of the lane's row and the horizontal chains pair up
+// the same way.  The masks are packed the same way.
 __device__ __forceinline__ uint32_t u16x2_max(uint32_t a, uint32_t b) {
   uint32_t r;
   asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
@@ -582,7 +585,7 @@ __device__ __forceinline__ uint32_t u16x2_min(uint32_t a, uint32_t b) {
   asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
-__device__ __forceinline__ uint32_t pk2(uint32_t lo, uint32_t hi) { return (lo & 0xffffu) | (hi << 16); }
+__device__ __forceinline__ uint32_t pk2(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x5410); }
 __device__ __forceinline__ uint32_t swap2(uint32_t x) { return __byte_perm(x, 0, 0x1032); }
 
 __device__ __forceinline__ uint32_t lds_u32(const uint32_t *p) {  // see lds_mask
@@ -592,36 +595,208 @@ __device__ __forceinline__ uint32_t lds_u32(const uint32_t *p) {  // see lds_mas
   return r;
 }
 
+
+// Shared memory of a packed tile's warp.  Rows of TP pixels are an odd number of words, so that a lane per row
+// and a lane per column both touch 32 banks.
+template <typename T> struct PackedTile {
+  static constexpr int TP = 32 + 4 / (int)sizeof(T);
+  uint32_t ma[16 * kRP];  // mask pairs of the rows (lane = column)
+  uint32_t mb[16 * kRP];  // mask pairs of the columns (lane = row)
+  T mask[32 * TP];
+  T val[32 * TP];         // staged values; transposes; write-back
+};
+
+// eight bytes from address a on, those outside the image at img zero, one by one (tiles at a buffer's ends)
+__device__ __noinline__ uint2 edge_bytes(uintptr_t a, const void *img, uintptr_t bytes) {
+  const uintptr_t base = reinterpret_cast<uintptr_t>(img);
+  uint32_t w[2] = {0u, 0u};
+  for (int b = 0; b < 8; ++b)
+    if (a + b >= base && a + b < base + bytes)
+      w[b >> 2] |= (uint32_t)*reinterpret_cast<const volatile unsigned char *>(a + b) << (8 * (b & 3));
+  return make_uint2(w[0], w[1]);
+}
+
+// One array of a tile in 8-byte pieces: pass k brings rows k * RI + lane / LR, piece lane % LR, at any
+// alignment: whole aligned words and a funnel shift with the next lane's.
+template <typename T, bool CG> struct TileRows {
+  static constexpr int LR = 4 * (int)sizeof(T), RI = 32 / LR, PASSES = 32 / RI;
+  const T *img;
+  uintptr_t a;       // this lane's piece of pass 0
+  intptr_t pitch;    // RI rows
+  bool safe, pairs;  // every word of the tile in the buffer; pieces aligned to 8 bytes
+  __device__ __forceinline__ TileRows(const void *img_, const RImg &im, int64_t y0, int64_t x0, int rows)
+      : img(static_cast<const T *>(img_)) {
+    const int lane = threadIdx.x & 31;
+    const intptr_t row = (intptr_t)im.W * (int)sizeof(T);
+    const uintptr_t base = reinterpret_cast<uintptr_t>(img), end = base + (uintptr_t)im.H * row;
+    const uintptr_t t = base + (uintptr_t)y0 * row + (uintptr_t)x0 * sizeof(T);
+    safe = (t & ~(uintptr_t)3) >= base && t + (rows - 1) * row + 8 * LR + 4 <= end;
+    pairs = ((t | (uintptr_t)row) & 7) == 0;
+    a = t + (lane / LR) * row + 8 * (lane % LR);
+    pitch = RI * row;
+  }
+  __device__ __forceinline__ static uint32_t ld(uintptr_t p) {
+    if constexpr (CG) return __ldcg(reinterpret_cast<const uint32_t *>(p));
+    else return __ldg(reinterpret_cast<const uint32_t *>(p));
+  }
+  // raw words of pass k: the piece's two aligned words and, in a row's last lane, the word after
+  __device__ __forceinline__ void load(int k, bool live, const RImg &im, uint32_t (&w)[3]) const {
+    const uintptr_t p = a + k * pitch;
+    w[0] = w[1] = w[2] = 0u;
+    if (!live) return;
+    if (!safe) {
+      const uint2 v = edge_bytes(p, img, (uintptr_t)(im.H * im.W) * sizeof(T));
+      w[0] = v.x;
+      w[1] = v.y;
+    } else if (pairs) {
+      uint2 v;
+      if constexpr (CG) v = __ldcg(reinterpret_cast<const uint2 *>(p));
+      else v = __ldg(reinterpret_cast<const uint2 *>(p));
+      w[0] = v.x;
+      w[1] = v.y;
+    } else {
+      const uintptr_t q = p & ~(uintptr_t)3;
+      w[0] = ld(q);
+      w[1] = ld(q + 4);
+      if ((threadIdx.x & 31) % LR == LR - 1) w[2] = ld(q + 8);
+    }
+  }
+  // the piece's pixels from its raw words; called by the whole warp
+  __device__ __forceinline__ uint2 pixels(int k, const uint32_t (&w)[3]) const {
+    if (!safe || pairs) return make_uint2(w[0], w[1]);  // uniform
+    const unsigned sh = (unsigned)((a + k * pitch) & 3u) * 8u;
+    uint32_t n = __shfl_down_sync(0xffffffffu, w[0], 1);
+    if ((threadIdx.x & 31) % LR == LR - 1) n = w[2];
+    return make_uint2(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], n, sh));
+  }
+};
+
+// One visit of a packed tile: as process_tile_reg below, but the pixels stay in their own width in shared memory
+// (6.5 KB a warp for u8, five CTAs per SM) and come in whole words at any alignment.  Rows of no whole 16-byte
+// vectors were staged pixel by pixel before: 21500 of a visit's 37700 cycles in a 512-image batch (sweeps 8100),
+// now 6600 of 22300; with the runs of for_pixel_runs and a search of the images in shared memory the batch of
+// 512 u8 images of 64-1024 pixels a side takes 2.37 ms (before: 6.25), one 2048^2 u8 image 131 us a call (177).
+// A visit is bound by latency: loads 6600 cycles, sweeps 7300, the fence, atomics and slot of its end 10300.
 template <typename T, bool SUP, bool CONN8>
-__device__ void sweeps_packed(T (&v)[32], RegS<T> *s_m, RegS<T> *s_t, int max_sweeps, T top, T bot, T hl, T hr,
-                              T initL, T initR, bool &converged, bool &changed, bool &wch, bool &ech) {
+__device__ __forceinline__ int process_tile_packed(const RImg &im, const RParams<T> &P, int t_local, PackedTile<T> &s) {
   static_assert(sizeof(T) <= 2, "two pixels per register");
+  constexpr int S = (int)sizeof(T), TP = PackedTile<T>::TP;
+  using OT = Op<T, SUP>;
+  constexpr int LR = TileRows<T, true>::LR, RI = TileRows<T, true>::RI, PASSES = TileRows<T, true>::PASSES;
   const int lane = threadIdx.x & 31;
+  const T NEU = OT::neutral();
+  const uint32_t NEUW = splat<T>(NEU);
+  const int tx = t_local % im.tiles_x, ty = t_local / im.tiles_x;
+  const int64_t y0 = (int64_t)ty * 32, x0 = (int64_t)tx * 32;
+  const int rows = (int)min((int64_t)32, im.H - y0), cols = (int)min((int64_t)32, im.W - x0);
+  const T *rec_in = static_cast<const T *>(im.rec);
+
+  // Halo, fixed during the visit: the row above and below per column, the columns left and right per row, and
+  // the four corners in lanes 0 (left) and 31 (right); outside the image the neutral value.
+  T h_top = NEU, h_bot = NEU, h_l = NEU, h_r = NEU, c_top = NEU, c_bot = NEU;
+  {
+    const T *top = rec_in + (y0 - 1) * im.W + x0, *bot = rec_in + (y0 + 32) * im.W + x0;
+    const T *left = rec_in + (y0 + lane) * im.W + x0 - 1;
+    const bool up = ty > 0, down = ty + 1 < im.tiles_y, west = tx > 0, east = tx + 1 < im.tiles_x;
+    if (up && lane < cols) h_top = ld_cg(top + lane);
+    if (down && lane < cols) h_bot = ld_cg(bot + lane);
+    if (west && lane < rows) h_l = ld_cg(left);
+    if (east && lane < rows) h_r = ld_cg(left + 33);
+    if (CONN8 && ((lane == 0 && west) || (lane == 31 && east))) {
+      const int c = lane == 0 ? -1 : 32;
+      if (up) c_top = ld_cg(top + c);
+      if (down) c_bot = ld_cg(bot + c);
+    }
+  }
+  // stage: the loads of four passes of both arrays go together
+  const TileRows<T, true> r_rec(im.rec, im, y0, x0, rows);
+  {
+    const TileRows<T, false> r_mask(im.mask, im, y0, x0, rows);
+#pragma unroll
+    for (int k0 = 0; k0 < PASSES; k0 += 4) {
+      uint32_t wm[4][3], wr[4][3];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool live = (k0 + k) * RI + lane / LR < rows;
+        r_mask.load(k0 + k, live, im, wm[k]);
+        r_rec.load(k0 + k, live, im, wr[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint2 m = r_mask.pixels(k0 + k, wm[k]), v = r_rec.pixels(k0 + k, wr[k]);
+        const int row = (k0 + k) * RI + lane / LR;
+        uint32_t *sm = reinterpret_cast<uint32_t *>(s.mask + row * TP) + 2 * (lane % LR);
+        uint32_t *sv = reinterpret_cast<uint32_t *>(s.val + row * TP) + 2 * (lane % LR);
+        sm[0] = m.x;
+        sm[1] = m.y;
+        sv[0] = v.x;
+        sv[1] = v.y;
+      }
+    }
+  }
+  if (needs_marker(P, 1)) {  // leveling: the effective mask
+    const TileRows<T, false> r_mark(im.marker, im, y0, x0, rows);
+#pragma unroll
+    for (int k0 = 0; k0 < PASSES; k0 += 4) {
+      uint32_t wk[4][3];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) r_mark.load(k0 + k, (k0 + k) * RI + lane / LR < rows, im, wk[k]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint2 b = r_mark.pixels(k0 + k, wk[k]);
+        uint32_t *sm = reinterpret_cast<uint32_t *>(s.mask + ((k0 + k) * RI + lane / LR) * TP) + 2 * (lane % LR);
+        if (P.mask_mode == MASK_MAX_MARKER) {
+          sm[0] = wop<T, true>(sm[0], b.x);
+          sm[1] = wop<T, true>(sm[1], b.y);
+        } else {
+          sm[0] = wop<T, false>(sm[0], b.x);
+          sm[1] = wop<T, false>(sm[1], b.y);
+        }
+      }
+    }
+  }
+  if (rows < 32 || cols < 32) {  // uniform: pixels outside the image are neutral
+#pragma unroll 1
+    for (int k = 0; k < PASSES; ++k) {
+      const int row = k * RI + lane / LR;
+      const int nb = row < rows ? min(max(cols * S - 8 * (lane % LR), 0), 8) : 0;
+      const unsigned long long in_m = nb == 8 ? ~0ull : (1ull << (8 * nb)) - 1ull;
+      uint32_t *sm = reinterpret_cast<uint32_t *>(s.mask + row * TP) + 2 * (lane % LR);
+      uint32_t *sv = reinterpret_cast<uint32_t *>(s.val + row * TP) + 2 * (lane % LR);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const uint32_t m = (uint32_t)(in_m >> (32 * j));
+        sm[j] = (sm[j] & m) | (NEUW & ~m);
+        sv[j] = (sv[j] & m) | (NEUW & ~m);
+      }
+    }
+  }
+  __syncwarp();
+  uint32_t V[16];
+#pragma unroll
+  for (int p = 0; p < 16; ++p) {
+    V[p] = pk2(s.val[p * TP + lane], s.val[(31 - p) * TP + lane]);
+    s.ma[p * kRP + lane] = pk2(s.mask[p * TP + lane], s.mask[(31 - p) * TP + lane]);
+    s.mb[p * kRP + lane] = pk2(s.mask[lane * TP + p], s.mask[lane * TP + 31 - p]);
+  }
+  // staged borders, to tell afterwards which neighbours must be revisited
+  const uint32_t init_tb = V[0], init_lr = pk2(s.val[lane * TP], s.val[lane * TP + 31]);
+  __syncwarp();
+  // a halo pixel's contribution goes into one value per border pixel (8-connected: the three beside it)
+  if (CONN8) {
+    auto up1 = [](T v, T first) { const T n = (T)__shfl_up_sync(0xffffffffu, (unsigned)v, 1); return (threadIdx.x & 31) == 0 ? first : n; };
+    auto dn1 = [](T v, T last) { const T n = (T)__shfl_down_sync(0xffffffffu, (unsigned)v, 1); return (threadIdx.x & 31) == 31 ? last : n; };
+    const T bl = (T)__shfl_sync(0xffffffffu, (unsigned)c_bot, 0), tr = (T)__shfl_sync(0xffffffffu, (unsigned)c_top, 31);
+    const T t3 = OT::apply(h_top, OT::apply(up1(h_top, c_top), dn1(h_top, c_top)));
+    const T b3 = OT::apply(h_bot, OT::apply(up1(h_bot, c_bot), dn1(h_bot, c_bot)));
+    const T l3 = OT::apply(h_l, OT::apply(up1(h_l, c_top), dn1(h_l, bl)));
+    const T r3 = OT::apply(h_r, OT::apply(up1(h_r, tr), dn1(h_r, c_bot)));
+    h_top = t3; h_bot = b3; h_l = l3; h_r = r3;
+  }
+  const uint32_t tb = pk2(h_top, h_bot), lr = pk2(h_l, h_r);
+
   auto OS = [](uint32_t a, uint32_t b) { return SUP ? u16x2_max(a, b) : u16x2_min(a, b); };  // propagation
   auto OC = [](uint32_t a, uint32_t b) { return SUP ? u16x2_min(a, b) : u16x2_max(a, b); };  // clip by the mask
-  // packed masks, rewritten over the unpacked ones: rows 0-15 of s_m hold the column pairs
-  // (lane = column), rows 16-31 the row pairs (lane = row)
-  uint32_t P[16];
-  {
-    uint32_t MA[16], MB[16];
-#pragma unroll
-    for (int p = 0; p < 16; ++p) {
-      MA[p] = pk2((uint32_t)s_m[p * kRP + lane], (uint32_t)s_m[(31 - p) * kRP + lane]);
-      MB[p] = pk2((uint32_t)s_m[lane * kRP + p], (uint32_t)s_m[lane * kRP + 31 - p]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int p = 0; p < 16; ++p) {
-      s_m[p * kRP + lane] = MA[p];
-      s_m[(16 + p) * kRP + lane] = MB[p];
-    }
-    __syncwarp();
-  }
-  const uint32_t *MAs = reinterpret_cast<const uint32_t *>(s_m) + lane;
-  const uint32_t *MBs = reinterpret_cast<const uint32_t *>(s_m) + 16 * kRP + lane;
-#pragma unroll
-  for (int p = 0; p < 16; ++p) P[p] = pk2(v[p], v[31 - p]);
-  const uint32_t tb = pk2(top, bot), lr = pk2(hl, hr);
   auto nbrow = [&](uint32_t x) -> uint32_t {
     if (CONN8) {
       const uint32_t a = __shfl_up_sync(0xffffffffu, x, 1), b = __shfl_down_sync(0xffffffffu, x, 1);
@@ -629,37 +804,38 @@ __device__ void sweeps_packed(T (&v)[32], RegS<T> *s_m, RegS<T> *s_t, int max_sw
     }
     return x;
   };
-  converged = false;
-  changed = false;
-  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+  const uint32_t *MAs = s.ma + lane, *MBs = s.mb + lane;
+  bool converged = false, changed = false;
+  uint32_t end_lr = init_lr;
+  for (int sweep = 0; sweep < P.max_sweeps; ++sweep) {
     uint32_t ch = 0;
-    // vertical: pair k from pair k - 1 (k = 0: the halo rows), then pair 15 from itself swapped
-    // and pair q from pair q + 1
+    // vertical: pair k from pair k - 1 (k = 0: the halo rows), then pair 15 from itself swapped and pair q
+    // from pair q + 1
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
-      const uint32_t nb = k == 0 ? tb : nbrow(P[k - 1]);  // the halo rows are already 3-wide
-      const uint32_t nv = OC(OS(P[k], nb), lds_u32(MAs + k * kRP));
-      ch |= nv ^ P[k];
-      P[k] = nv;
+      const uint32_t nb = k == 0 ? tb : nbrow(V[k - 1]);  // the halo rows are already 3-wide
+      const uint32_t nv = OC(OS(V[k], nb), lds_u32(MAs + k * kRP));
+      ch |= nv ^ V[k];
+      V[k] = nv;
     }
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
       const int q = 15 - k;
-      const uint32_t nb = nbrow(k == 0 ? swap2(P[15]) : P[q + 1]);
-      const uint32_t nv = OC(OS(P[q], nb), lds_u32(MAs + q * kRP));
-      ch |= nv ^ P[q];
-      P[q] = nv;
+      const uint32_t nb = nbrow(k == 0 ? swap2(V[15]) : V[q + 1]);
+      const uint32_t nv = OC(OS(V[q], nb), lds_u32(MAs + q * kRP));
+      ch |= nv ^ V[q];
+      V[q] = nv;
     }
     // to lane = row
 #pragma unroll
     for (int p = 0; p < 16; ++p) {
-      s_t[p * kRP + lane] = P[p] & 0xffffu;
-      s_t[(31 - p) * kRP + lane] = P[p] >> 16;
+      s.val[p * TP + lane] = (T)V[p];
+      s.val[(31 - p) * TP + lane] = (T)(V[p] >> 16);
     }
     __syncwarp();
     uint32_t Q[16];
 #pragma unroll
-    for (int c = 0; c < 16; ++c) Q[c] = pk2((uint32_t)s_t[lane * kRP + c], (uint32_t)s_t[lane * kRP + 31 - c]);
+    for (int c = 0; c < 16; ++c) Q[c] = pk2(s.val[lane * TP + c], s.val[lane * TP + 31 - c]);
     __syncwarp();
     // horizontal, the same pairing
 #pragma unroll
@@ -677,29 +853,57 @@ __device__ void sweeps_packed(T (&v)[32], RegS<T> *s_m, RegS<T> *s_t, int max_sw
       ch |= nv ^ Q[q];
       Q[q] = nv;
     }
-    wch = (T)(Q[0] & 0xffffu) != initL;
-    ech = (T)(Q[0] >> 16) != initR;
-    // back to lane = column
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      s_t[lane * kRP + c] = Q[c] & 0xffffu;
-      s_t[lane * kRP + 31 - c] = Q[c] >> 16;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int p = 0; p < 16; ++p) P[p] = pk2((uint32_t)s_t[p * kRP + lane], (uint32_t)s_t[(31 - p) * kRP + lane]);
-    __syncwarp();
+    end_lr = Q[0];
     if (!__any_sync(0xffffffffu, ch != 0)) {
-      converged = true;
+      converged = true;  // nothing moved: V still holds the values
       break;
     }
     changed = true;
-  }
+    // back to lane = column
 #pragma unroll
-  for (int p = 0; p < 16; ++p) {
-    v[p] = (T)(P[p] & 0xffffu);
-    v[31 - p] = (T)(P[p] >> 16);
+    for (int c = 0; c < 16; ++c) {
+      s.val[lane * TP + c] = (T)Q[c];
+      s.val[lane * TP + 31 - c] = (T)(Q[c] >> 16);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int p = 0; p < 16; ++p) V[p] = pk2(s.val[p * TP + lane], s.val[(31 - p) * TP + lane]);
+    __syncwarp();
   }
+
+  const uint32_t d_tb = V[0] ^ init_tb, d_lr = end_lr ^ init_lr;
+  const unsigned bN = __ballot_sync(0xffffffffu, (d_tb & 0xffffu) != 0u), bS = __ballot_sync(0xffffffffu, (d_tb >> 16) != 0u);
+  const unsigned bW = __ballot_sync(0xffffffffu, (d_lr & 0xffffu) != 0u), bE = __ballot_sync(0xffffffffu, (d_lr >> 16) != 0u);
+  int f = converged ? 0 : B_SELF;
+  if (bN) f |= B_N;
+  if (bS) f |= B_S;
+  if (bW) f |= B_W;
+  if (bE) f |= B_E;
+  if (bN & 1u) f |= B_NW;
+  if (bN >> 31) f |= B_NE;
+  if (bS & 1u) f |= B_SW;
+  if (bS >> 31) f |= B_SE;
+
+  if (changed) {
+    T *rec = static_cast<T *>(im.rec);
+    if (r_rec.pairs && cols == 32) {
+      // s.val holds the last values by rows (the transposes leave them there): 8-byte pieces out
+#pragma unroll
+      for (int k = 0; k < PASSES; ++k) {
+        const int row = k * RI + lane / LR;
+        const uint32_t *sv = reinterpret_cast<const uint32_t *>(s.val + row * TP) + 2 * (lane % LR);
+        if (row < rows) __stcg(reinterpret_cast<uint2 *>(r_rec.a + k * r_rec.pitch), make_uint2(sv[0], sv[1]));
+      }
+    } else if (lane < cols) {
+      T *p = rec + y0 * im.W + x0 + lane;
+#pragma unroll
+      for (int r = 0; r < 32; ++r) {
+        if (r < rows) st_cg(p + r * im.W, (T)(r < 16 ? V[r] : V[31 - r] >> 16));
+      }
+    }
+    __syncwarp();
+  }
+  return f;
 }
 
 // One visit of a register tile: stage it from the reconstruction buffer (which the worklist
@@ -707,7 +911,7 @@ __device__ void sweeps_packed(T (&v)[32], RegS<T> *s_m, RegS<T> *s_t, int max_sw
 // P.max_sweeps), write it back if anything changed.  Returns the B_* bits of the borders that
 // changed (the neighbours to revisit) and B_SELF when the tile yielded.  Warp-uniform.
 template <typename T, bool SUP, bool CONN8>
-__device__ int process_tile_reg(const RImg &im, const RParams<T> &P, int t_local, RegS<T> *s_m, RegS<T> *s_t) {
+__device__ int process_tile_reg(const RImg &im, const RParams<T> &P, int t_local, T *s_m, T *s_t) {
   using OS = Op<T, SUP>;   // propagation
   using OC = Op<T, !SUP>;  // clip by the mask
   const int lane = threadIdx.x & 31;
@@ -741,44 +945,7 @@ __device__ int process_tile_reg(const RImg &im, const RParams<T> &P, int t_local
   const T *ms_in = static_cast<const T *>(im.mask);
   const bool need_mk = needs_marker(P, 1);
   T v[32];
-  bool vec = false;
-  if constexpr (sizeof(T) <= 2) {
-    // rows of whole 16-byte vectors: the tile (32 rows x 32 or 64 bytes) comes in 2 * sizeof(T)
-    // vector loads per lane and array, unpacked into shared memory; v is then read per column
-    vec = (im.W * (int64_t)sizeof(T)) % 16 == 0 &&
-          ((reinterpret_cast<uintptr_t>(ms_in) | reinterpret_cast<uintptr_t>(rec_in) |
-            (need_mk ? reinterpret_cast<uintptr_t>(mk_in) : (uintptr_t)0)) % 16) == 0;
-  }
-  if (vec) {
-    constexpr int VPR = 2 * (int)sizeof(T);   // 16-byte vectors per tile row
-    constexpr int VPX = 16 / (int)sizeof(T);  // pixels per vector
-    uint4 ma[VPR], ka[VPR], ra[VPR];
-#pragma unroll
-    for (int k = 0; k < VPR; ++k) {
-      const int q = k * 32 + lane, row = q / VPR, vc = q % VPR;
-      const int64_t gy = y0 + row, gx0 = x0 + vc * VPX;
-      const int64_t gi = (gy < im.H && gx0 < im.W) ? gy * im.W + gx0 : 0;
-      ma[k] = __ldg(reinterpret_cast<const uint4 *>(ms_in + gi));
-      ka[k] = need_mk ? __ldg(reinterpret_cast<const uint4 *>(mk_in + gi)) : ma[k];
-      ra[k] = __ldcg(reinterpret_cast<const uint4 *>(rec_in + gi));
-    }
-#pragma unroll
-    for (int k = 0; k < VPR; ++k) {
-      const int q = k * 32 + lane, row = q / VPR, vc = q % VPR;
-      const bool ok = y0 + row < im.H && x0 + vc * VPX < im.W;
-#pragma unroll
-      for (int e = 0; e < VPX; ++e) {
-        const T a = vec_elem<T>(ma[k], e), b = vec_elem<T>(ka[k], e), c = vec_elem<T>(ra[k], e);
-        s_m[row * kRP + vc * VPX + e] = ok ? combine_mask(P, a, b) : NEU;
-        s_t[row * kRP + vc * VPX + e] = ok ? c : NEU;
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < 32; ++r) v[r] = (T)s_t[r * kRP + lane];
-    __syncwarp();
-  } else {
-  // scalar stage: loads come first, 16 rows at a time, so that they are all in flight together
+  // loads come first, 16 rows at a time, so that they are all in flight together
 #pragma unroll
   for (int h = 0; h < 32; h += 16) {
     T a[16], b[16];
@@ -801,7 +968,6 @@ __device__ int process_tile_reg(const RImg &im, const RParams<T> &P, int t_local
       s_m[(h + r) * kRP + lane] = m;
     }
   }
-  }
   T top = hv[0], bot = hv[1], hl = hv[2], hr = hv[3];
   if (CONN8) {
     top = OS::apply(top, OS::apply(hv[4], hv[5]));
@@ -818,9 +984,6 @@ __device__ int process_tile_reg(const RImg &im, const RParams<T> &P, int t_local
   __syncwarp();
 
   bool converged = false, changed = false, wch = false, ech = false;
-  if constexpr (sizeof(T) <= 2) {
-    sweeps_packed<T, SUP, CONN8>(v, s_m, s_t, P.max_sweeps, top, bot, hl, hr, initL, initR, converged, changed, wch, ech);
-  } else {
   for (int sweep = 0; sweep < P.max_sweeps; ++sweep) {
     bool ch = false;
     auto vstep = [&](int r, T nb) {
@@ -891,7 +1054,6 @@ __device__ int process_tile_reg(const RImg &im, const RParams<T> &P, int t_local
     changed = true;
   }
 
-  }
   const unsigned bN = __ballot_sync(0xffffffffu, v[0] != initT);
   const unsigned bS = __ballot_sync(0xffffffffu, v[31] != initB);
   const unsigned bW = __ballot_sync(0xffffffffu, wch);
@@ -906,31 +1068,7 @@ __device__ int process_tile_reg(const RImg &im, const RParams<T> &P, int t_local
   if (bS & 1u) f |= B_SW;
   if (bS >> 31) f |= B_SE;
 
-  if (changed && vec) {
-    // the stage's vector layout in reverse: columns to shared memory, rows out as 16-byte stores
-    if constexpr (sizeof(T) <= 2) {
-      constexpr int VPR = 2 * (int)sizeof(T), VPX = 16 / (int)sizeof(T), PW = 4 / (int)sizeof(T);
-#pragma unroll
-      for (int r = 0; r < 32; ++r) s_t[r * kRP + lane] = v[r];
-      __syncwarp();
-      T *rec = static_cast<T *>(im.rec);
-#pragma unroll
-      for (int k = 0; k < VPR; ++k) {
-        const int q = k * 32 + lane, row = q / VPR, vc = q % VPR;
-        const int64_t gy = y0 + row, gx0 = x0 + vc * VPX;
-        uint32_t w[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          w[j] = 0u;
-#pragma unroll
-          for (int e = 0; e < PW; ++e)
-            w[j] |= ((uint32_t)s_t[row * kRP + vc * VPX + j * PW + e] & Lim<T>::hi()) << (8 * (int)sizeof(T) * e);
-        }
-        if (gy < im.H && gx0 < im.W) __stcg(reinterpret_cast<uint4 *>(rec + gy * im.W + gx0), make_uint4(w[0], w[1], w[2], w[3]));
-      }
-      __syncwarp();
-    }
-  } else if (changed) {
+  if (changed) {
     // the row stride goes through a shuffle so that the compiler recomputes these addresses
     // here instead of keeping the stage's 32 row addresses alive across the sweeps
     const long long Wd = __shfl_sync(0xffffffffu, (long long)im.W, 0);
@@ -992,30 +1130,34 @@ __device__ __forceinline__ unsigned long long slot_val(unsigned pos, unsigned ti
   return ((unsigned long long)pos << 32) | tile1;
 }
 
-// Lane 0 pops: the tile to visit, or -1 when the work is done or an error was recorded.
+// Lane 0 pops ticket `pos`: the tile to visit, or -1 when the work is done or an error was recorded.  A waiting
+// warp polls its own slot only (every idle warp polling the shared counters as well slowed the atomics on
+// them): the warp that ends the last visit fills the slots of the tickets still out with kExit, and a warp that
+// takes its ticket later sees `pending` at zero on its first poll.
+static constexpr unsigned kExit = 0xffffffffu;
+
 template <typename T>
-__device__ int wl_pop(const WorkList<T> &wl, RCtl *ctl, long long max_tickets) {
-  const unsigned pos = atomicAdd(&wl.q->head, 1u);
+__device__ int wl_pop(const WorkList<T> &wl, RCtl *ctl, unsigned pos, long long max_tickets) {
   if ((long long)pos >= max_tickets) {  // runaway guard: far more visits than any input needs
     set_status(ctl, PG_ERR_NOT_CONVERGED);
     return -1;
   }
   volatile unsigned long long *slot = wl.ring + pos % wl.cap;
   const unsigned long long t0 = global_ns();
-  unsigned ns = 32;
   unsigned long long v;
-  for (;;) {
-    // the three words are read together (one memory round trip per poll, not three in a row)
+  for (unsigned polls = 0;; ++polls) {
     v = *slot;
-    const unsigned long long tp = *((volatile unsigned long long *)&wl.q->tp);
-    const int st = *((volatile int *)&ctl->status);
+    unsigned long long tp = ~0ull;
+    if (polls % 16 == 0) tp = *((volatile unsigned long long *)&wl.q->tp);  // with the slot: one round trip
     if ((unsigned)(v >> 32) == pos && (unsigned)v != 0u) break;
     if (tp_pending(tp) == 0) return -1;
-    if (st != 0) return -1;
-    __nanosleep(ns);
-    if (ns < 1024) ns <<= 1;  // longest back-off 1 us: measured 6 % faster than 4 us on the h-maxima input
-    if (wait_expired(ctl, t0, wl.wait_ns)) return -1;
+    if (polls % 16 == 15) {
+      if (*((volatile int *)&ctl->status) != 0) return -1;
+      if (wait_expired(ctl, t0, wl.wait_ns)) return -1;
+    }
+    __nanosleep(polls < 8 ? 40 : 200);
   }
+  if ((unsigned)v == kExit) return -1;
   *slot = slot_val(pos, 0u);  // consumed: the next lap's pusher may write
   const unsigned tile = (unsigned)v - 1u;
   *((volatile unsigned *)(wl.state + tile)) = TS_RUNNING;  // QUEUED until now: nobody else moves it
@@ -1046,38 +1188,46 @@ __device__ void wl_finish(const WorkList<T> &wl, RCtl *ctl, const RImg &im, int 
     const int nx = tx + dx, ny = ty + dy;
     if (nx >= 0 && ny >= 0 && nx < im.tiles_x && ny < im.tiles_y) cand = im.tile_begin + ny * im.tiles_x + nx;
   }
+  // Every lane's expected transition in one compare-and-swap, all in flight together; what another warp moved
+  // in between is settled after.
+  const bool self = lane == 8, yielded = (f & B_SELF) != 0;
+  if (self) cand = tile;
   if (cand >= 0) {
+    unsigned want = self ? TS_RUNNING : TS_IDLE, to = self && !yielded ? TS_IDLE : TS_QUEUED;
     bool done = false;
     for (int it = 0; it < kCasRetries && !done; ++it) {
-      const unsigned s = atomicCAS(wl.state + cand, TS_IDLE, TS_QUEUED);
-      if (s == TS_IDLE) push = done = true;
-      else if (s != TS_RUNNING) done = true;  // already queued, or already marked for another visit
-      else if (atomicCAS(wl.state + cand, TS_RUNNING, TS_DIRTY) == TS_RUNNING) done = true;
-    }
-    if (!done) set_status(ctl, PG_ERR_NOT_CONVERGED);
-  }
-  if (lane == 8) {
-    // release: back to IDLE, or queued again if it yielded or a neighbour changed meanwhile
-    const bool yielded = (f & B_SELF) != 0;
-    bool done = false;
-    for (int it = 0; it < kCasRetries && !done; ++it) {
-      const unsigned s = *((volatile unsigned *)(wl.state + tile));  // RUNNING or DIRTY: only we move it out
-      if (s == TS_DIRTY || yielded) {
-        if (atomicCAS(wl.state + tile, s, TS_QUEUED) == s) push = done = true;
-      } else if (atomicCAS(wl.state + tile, TS_RUNNING, TS_IDLE) == TS_RUNNING) {
+      const unsigned s = atomicCAS(wl.state + cand, want, to);
+      if (s == want) {
+        push = to == TS_QUEUED;
         done = true;
+      } else if (self) {  // DIRTY: a neighbour changed its border meanwhile; only we move it out
+        want = s;
+        to = TS_QUEUED;
+      } else if (s == TS_RUNNING) {
+        want = TS_RUNNING;
+        to = TS_DIRTY;
+      } else if (s == TS_IDLE) {
+        want = TS_IDLE;
+        to = TS_QUEUED;
+      } else {
+        done = true;  // already queued, or already marked for another visit
       }
     }
     if (!done) set_status(ctl, PG_ERR_NOT_CONVERGED);
-    cand = tile;
   }
   const unsigned pm = __ballot_sync(0xffffffffu, push);
+  // One atomic reserves the pushed tiles' positions, counts them and takes this visit off `pending`: a tile
+  // cannot be popped and finished before it is counted, so `pending` is zero only when all work is done.
   const int n = __popc(pm);
-  unsigned base = 0;
-  if (lane == 0 && n > 0) {
-    base = tp_tail(atomicAdd(&wl.q->tp, ((unsigned long long)n << 32) | (unsigned long long)n));
+  unsigned base = 0, left = 0;
+  if (lane == 0) {
+    const unsigned long long add = ((unsigned long long)(unsigned)(n - 1) << 32) + (unsigned)n;
+    const unsigned long long tp = atomicAdd(&wl.q->tp, add);
+    base = tp_tail(tp);
+    left = (unsigned)tp_pending(tp + add);
   }
   base = __shfl_sync(0xffffffffu, base, 0);
+  left = __shfl_sync(0xffffffffu, left, 0);
   if (push) {
     const unsigned pos = base + __popc(pm & ((1u << lane) - 1u));
     volatile unsigned long long *slot = wl.ring + pos % wl.cap;
@@ -1092,61 +1242,100 @@ __device__ void wl_finish(const WorkList<T> &wl, RCtl *ctl, const RImg &im, int 
     }
     *slot = slot_val(pos, (unsigned)cand + 1u);
   }
-  // pending - 1, after this warp's pushes were counted (same word, same thread): never 0 early
-  if (lane == 0) atomicAdd(&wl.q->tp, ~0ull << 32);
+  if (left == 0) {  // the last visit: release the warps that wait (tickets from the tail on)
+    unsigned head = 0;
+    if (lane == 0) {
+      __threadfence();  // a ticket taken after this read finds `pending` at zero
+      head = atomicAdd(&wl.q->head, 0u);
+    }
+    head = __shfl_sync(0xffffffffu, head, 0);
+    for (unsigned pos = base + (unsigned)n + lane; (int)(head - pos) > 0; pos += 32)
+      *((volatile unsigned long long *)(wl.ring + pos % wl.cap)) = slot_val(pos, kExit);
+  }
 }
 
-// first phase: every reconstruction buffer starts at the marker (select_marker, or the
-// saturated shift of the h-extrema), EPI_UNROLL pixels per thread and step
+// first phase: every reconstruction buffer starts at the marker (select_marker, or the saturated shift of the
+// h-extrema)
 template <typename T, bool SUP>
-__device__ void init_rec(const RParams<T> &P, int64_t tid, int64_t nth) {
+__device__ void init_rec(const RParams<T> &P, const int *begin) {
   const bool need_mk = needs_marker(P, 0);
-  for (int k = 0; k < P.nimg; ++k) {
-    const RImg &im = (P.nimg == 1) ? P.single : P.imgs[k];
-    const int64_t n = im.H * im.W;
+  const int lane = threadIdx.x & 31;
+  for_pixel_runs(P, begin, [&](const RImg &im, int64_t lo, int64_t hi) {
     const T *ms = static_cast<const T *>(im.mask);
-    const T *mk = static_cast<const T *>(im.marker);
+    const T *mk = need_mk ? static_cast<const T *>(im.marker) : ms;
     T *rec = static_cast<T *>(im.rec);
-    for (int64_t i0 = tid; i0 < n; i0 += nth * EPI_UNROLL) {
+    constexpr int VE = Pack<T>::N;
+    int64_t done = lo;
+    if ((reinterpret_cast<uintptr_t>(ms) | reinterpret_cast<uintptr_t>(mk) | reinterpret_cast<uintptr_t>(rec)) % 16 == 0) {
+#pragma unroll 2
+      for (int64_t j = lo / VE + lane; j < hi / VE; j += 32) {
+        const Pack<T> a = Pack<T>::load(ms + j * VE), b = need_mk ? Pack<T>::load(mk + j * VE) : a;
+        Pack<T> r;
+#pragma unroll
+        for (int e = 0; e < VE; ++e) {
+          T m;
+          combine_init<T, SUP>(P, a.e[e], b.e[e], m, r.e[e]);
+        }
+        __stcg(reinterpret_cast<uint4 *>(rec + j * VE), r.v);
+      }
+      done = hi / VE * VE;
+    }
+    for (int64_t i0 = done + lane; i0 < hi; i0 += 32 * EPI_UNROLL) {
       T a[EPI_UNROLL], b[EPI_UNROLL];
 #pragma unroll
       for (int u = 0; u < EPI_UNROLL; ++u) {
-        const int64_t i = i0 + u * nth;
-        a[u] = i < n ? ldg(ms + i) : T(0);
-        b[u] = (need_mk && i < n) ? ldg(mk + i) : a[u];
+        const int64_t i = i0 + u * 32;
+        a[u] = i < hi ? ldg(ms + i) : T(0);
+        b[u] = (need_mk && i < hi) ? ldg(mk + i) : a[u];
       }
 #pragma unroll
       for (int u = 0; u < EPI_UNROLL; ++u) {
-        const int64_t i = i0 + u * nth;
+        const int64_t i = i0 + u * 32;
         T m, v;
         combine_init<T, SUP>(P, a[u], b[u], m, v);
-        if (i < n) st_cg(rec + i, v);
+        if (i < hi) st_cg(rec + i, v);
       }
     }
-  }
+  });
 }
 
 __device__ long long g_recon_visits = 0;
 
+template <typename T> struct TileSmem {
+  static constexpr size_t bytes = 2 * 32 * kRP * sizeof(T);  // process_tile_reg's two arrays
+};
+template <> struct TileSmem<uint8_t> { static constexpr size_t bytes = (sizeof(PackedTile<uint8_t>) + 15) / 16 * 16; };
+template <> struct TileSmem<uint16_t> { static constexpr size_t bytes = (sizeof(PackedTile<uint16_t>) + 15) / 16 * 16; };
+constexpr int kBeginMax = 1024;  // images whose first tiles are kept in shared memory
+
 template <typename T, bool SUP, bool CONN8>
-__global__ void __launch_bounds__(kRegWarps * 32, 4) k_reconstruct_wl(RParams<T> P, WorkList<T> wl) {
+__global__ void __launch_bounds__(kRegWarps * 32, sizeof(T) <= 2 ? 5 : 4) k_reconstruct_wl(const __grid_constant__ RParams<T> P,
+                                                                                          const WorkList<T> wl) {
   static_assert(sizeof(T) <= 4, "register tiles hold pixels of at most 4 bytes");
-  __shared__ RegS<T> s_m[kRegWarps][32 * kRP];
-  __shared__ RegS<T> s_t[kRegWarps][32 * kRP];
+  __shared__ __align__(16) unsigned char s_raw[kRegWarps][TileSmem<T>::bytes];
+  __shared__ int s_begin[kBeginMax];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   RCtl *ctl = P.ctl;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nth = (int64_t)gridDim.x * blockDim.x;
 
+  // the images' first tiles, for the searches of image_of
+  const int *begin = P.nimg > 1 && P.nimg <= kBeginMax ? s_begin : nullptr;
+  if (begin) {
+    for (int k = threadIdx.x; k < P.nimg; k += blockDim.x) s_begin[k] = P.imgs[k].tile_begin;
+    __syncthreads();
+  }
   // phase 0: marker into the reconstruction buffers, every tile queued once
-  init_rec<T, SUP>(P, tid, nth);
+  init_rec<T, SUP>(P, begin);
   for (int64_t i = tid; i < (int64_t)wl.cap; i += nth) {
     // positions 0..ntiles-1 hold the tiles; the others wait for their first lap
     wl.ring[i] = i < P.ntiles ? slot_val((unsigned)i, (unsigned)i + 1u) : slot_val((unsigned)i - wl.cap, 0u);
     if (i < P.ntiles) wl.state[i] = TS_QUEUED;
   }
+  const unsigned warps = (unsigned)(nth >> 5);
   if (tid == 0) {
     wl.q->tp = ((unsigned long long)P.ntiles << 32) | (unsigned long long)P.ntiles;
+    wl.q->head = warps;  // every warp starts with the ticket of its number
   }
   if (!grid_barrier(ctl, P.wait_ns)) return;
 
@@ -1154,17 +1343,24 @@ __global__ void __launch_bounds__(kRegWarps * 32, 4) k_reconstruct_wl(RParams<T>
   // runaway guard on the tickets (visits plus idle pops), also below the wrap of the 32-bit ring
   // positions
   const long long max_tickets = std::min<long long>((long long)P.ntiles * P.max_rounds, (1ll << 31) - 2ll * P.ntiles);
-  for (;;) {
+  for (unsigned ticket = (unsigned)(tid >> 5);;) {
     int t = -1;
-    if (lane == 0) t = wl_pop(wl, ctl, max_tickets);
+    if (lane == 0) t = wl_pop(wl, ctl, ticket, max_tickets);
     t = __shfl_sync(0xffffffffu, t, 0);
     if (t < 0) break;
     int tl = 0;
-    const RImg &im = image_of(P, t, tl);
-    const int f = process_tile_reg<T, SUP, CONN8>(im, P, tl, s_m[warp], s_t[warp]);
+    const RImg &im = image_of(P, t, tl, begin);
+    int f;
+    if constexpr (sizeof(T) <= 2) {
+      f = process_tile_packed<T, SUP, CONN8>(im, P, tl, *reinterpret_cast<PackedTile<T> *>(s_raw[warp]));
+    } else {
+      T *s_m = reinterpret_cast<T *>(s_raw[warp]);
+      f = process_tile_reg<T, SUP, CONN8>(im, P, tl, s_m, s_m + 32 * kRP);
+    }
     __threadfence();  // this tile's pixels, before any neighbour is queued
     __syncwarp();
     wl_finish<T, CONN8>(wl, ctl, im, t, tl, f);
+    if (lane == 0) ticket = atomicAdd(&wl.q->head, 1u);
     __syncwarp();
   }
   if (!grid_barrier(ctl, P.wait_ns)) return;
@@ -1175,7 +1371,7 @@ __global__ void __launch_bounds__(kRegWarps * 32, 4) k_reconstruct_wl(RParams<T>
     ctl->rounds = g_recon_rounds;
   }
   if (P.epi == EPI_NONE) return;
-  recon_epilogue<T, SUP>(P);
+  recon_epilogue<T, SUP>(P, begin);
 }
 
 // ------------------------------------------------------------------ host side
