@@ -10,7 +10,9 @@
 // with mask max(marker, ref) (low) / min(marker, ref) (high) followed by a clip by ref.
 //
 // GPU design: tiles iterated to a tile-local fixpoint, scheduled until no tile changes.
-//  * Pixels of at most 4 bytes (k_reconstruct_wl): 32x32 tiles, one warp per tile, the tile
+//  * Single images of 1- or 2-byte pixels whose 32x32 tiles all fit on the GPU at once
+//    (k_reconstruct_resident): every tile stays in its warp, neighbours exchange border pixels.
+//  * Other images of pixels of at most 4 bytes (k_reconstruct_wl): 32x32 tiles, one warp per tile, the tile
 //    in registers; directional sweep sets (down/up by warp shuffles, right/left after a
 //    shared-memory transpose; two rows per register for 1- and 2-byte pixels) until a set
 //    changes nothing.  The tiles are driven by a device worklist (a ticket ring and a state
@@ -598,12 +600,14 @@ __device__ __forceinline__ uint32_t lds_u32(const uint32_t *p) {  // see lds_mas
 
 // Shared memory of a packed tile's warp.  Rows of TP pixels are an odd number of words, so that a lane per row
 // and a lane per column both touch 32 banks.
-template <typename T> struct PackedTile {
+template <typename T> struct PackedCore {
   static constexpr int TP = 32 + 4 / (int)sizeof(T);
   uint32_t ma[16 * kRP];  // mask pairs of the rows (lane = column)
   uint32_t mb[16 * kRP];  // mask pairs of the columns (lane = row)
-  T mask[32 * TP];
   T val[32 * TP];         // staged values; transposes; write-back
+};
+template <typename T> struct PackedTile : PackedCore<T> {
+  T mask[32 * PackedCore<T>::TP];  // staged mask
 };
 
 // eight bytes from address a on, those outside the image at img zero, one by one (tiles at a buffer's ends)
@@ -670,6 +674,113 @@ template <typename T, bool CG> struct TileRows {
     return make_uint2(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], n, sh));
   }
 };
+
+// Sweep sets of a packed tile until one changes nothing (returns true) or max_sweeps of them ran.  V: row pairs
+// (lane = column), in and out; tb, lr: what the halo contributes to the first pair of each direction; end_lr:
+// the outermost column pair (lane = row) at the end.  s.val is overwritten: where a set changed something it
+// holds the last values by rows.
+template <typename T, bool SUP, bool CONN8>
+__device__ __forceinline__ bool packed_sweeps(uint32_t (&V)[16], PackedCore<T> &s, uint32_t tb, uint32_t lr, int max_sweeps,
+                                              uint32_t &end_lr, bool &changed) {
+  constexpr int TP = PackedCore<T>::TP;
+  const int lane = threadIdx.x & 31;
+  auto OS = [](uint32_t a, uint32_t b) { return SUP ? u16x2_max(a, b) : u16x2_min(a, b); };  // propagation
+  auto OC = [](uint32_t a, uint32_t b) { return SUP ? u16x2_min(a, b) : u16x2_max(a, b); };  // clip by the mask
+  auto nbrow = [&](uint32_t x) -> uint32_t {
+    if (CONN8) {
+      const uint32_t a = __shfl_up_sync(0xffffffffu, x, 1), b = __shfl_down_sync(0xffffffffu, x, 1);
+      return OS(x, OS(a, b));
+    }
+    return x;
+  };
+  const uint32_t *MAs = s.ma + lane, *MBs = s.mb + lane;
+  changed = false;
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    uint32_t ch = 0;
+    // vertical: pair k from pair k - 1 (k = 0: the halo rows), then pair 15 from itself swapped and pair q
+    // from pair q + 1
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const uint32_t nb = k == 0 ? tb : nbrow(V[k - 1]);  // the halo rows are already 3-wide
+      const uint32_t nv = OC(OS(V[k], nb), lds_u32(MAs + k * kRP));
+      ch |= nv ^ V[k];
+      V[k] = nv;
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const int q = 15 - k;
+      const uint32_t nb = nbrow(k == 0 ? swap2(V[15]) : V[q + 1]);
+      const uint32_t nv = OC(OS(V[q], nb), lds_u32(MAs + q * kRP));
+      ch |= nv ^ V[q];
+      V[q] = nv;
+    }
+    // to lane = row
+#pragma unroll
+    for (int p = 0; p < 16; ++p) {
+      s.val[p * TP + lane] = (T)V[p];
+      s.val[(31 - p) * TP + lane] = (T)(V[p] >> 16);
+    }
+    __syncwarp();
+    uint32_t Q[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) Q[c] = pk2(s.val[lane * TP + c], s.val[lane * TP + 31 - c]);
+    __syncwarp();
+    // horizontal, the same pairing
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const uint32_t nb = k == 0 ? lr : Q[k - 1];
+      const uint32_t nv = OC(OS(Q[k], nb), lds_u32(MBs + k * kRP));
+      ch |= nv ^ Q[k];
+      Q[k] = nv;
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const int q = 15 - k;
+      const uint32_t nb = k == 0 ? swap2(Q[15]) : Q[q + 1];
+      const uint32_t nv = OC(OS(Q[q], nb), lds_u32(MBs + q * kRP));
+      ch |= nv ^ Q[q];
+      Q[q] = nv;
+    }
+    end_lr = Q[0];
+    const bool any = __any_sync(0xffffffffu, ch != 0);
+    changed |= any;
+    // back to lane = column (where nothing moved, s.val still holds the values by rows)
+    if (any) {
+#pragma unroll
+      for (int c = 0; c < 16; ++c) {
+        s.val[lane * TP + c] = (T)Q[c];
+        s.val[lane * TP + 31 - c] = (T)(Q[c] >> 16);
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int p = 0; p < 16; ++p) V[p] = pk2(s.val[p * TP + lane], s.val[(31 - p) * TP + lane]);
+    __syncwarp();
+    if (!any) return true;
+  }
+  return false;
+}
+
+// A halo pixel's contribution goes into one value per border pixel; 8-connected: of the three pixels beside it.
+// h_top, h_bot: per column; h_l, h_r: per row; c_top, c_bot: the corners, left ones in lane 0, right in lane 31.
+template <typename T, bool SUP>
+__device__ __forceinline__ void fold_halo(T &h_top, T &h_bot, T &h_l, T &h_r, T c_top, T c_bot) {
+  using OT = Op<T, SUP>;
+  auto up1 = [](T v, T first) {
+    const T n = (T)__shfl_up_sync(0xffffffffu, (unsigned)v, 1);
+    return (threadIdx.x & 31) == 0 ? first : n;
+  };
+  auto dn1 = [](T v, T last) {
+    const T n = (T)__shfl_down_sync(0xffffffffu, (unsigned)v, 1);
+    return (threadIdx.x & 31) == 31 ? last : n;
+  };
+  const T bl = (T)__shfl_sync(0xffffffffu, (unsigned)c_bot, 0), tr = (T)__shfl_sync(0xffffffffu, (unsigned)c_top, 31);
+  const T t3 = OT::apply(h_top, OT::apply(up1(h_top, c_top), dn1(h_top, c_top)));
+  const T b3 = OT::apply(h_bot, OT::apply(up1(h_bot, c_bot), dn1(h_bot, c_bot)));
+  const T l3 = OT::apply(h_l, OT::apply(up1(h_l, c_top), dn1(h_l, bl)));
+  const T r3 = OT::apply(h_r, OT::apply(up1(h_r, tr), dn1(h_r, c_bot)));
+  h_top = t3; h_bot = b3; h_l = l3; h_r = r3;
+}
 
 // One visit of a packed tile: as process_tile_reg below, but the pixels stay in their own width in shared memory
 // (6.5 KB a warp for u8, five CTAs per SM) and come in whole words at any alignment.  Rows of no whole 16-byte
@@ -782,94 +893,12 @@ __device__ __forceinline__ int process_tile_packed(const RImg &im, const RParams
   // staged borders, to tell afterwards which neighbours must be revisited
   const uint32_t init_tb = V[0], init_lr = pk2(s.val[lane * TP], s.val[lane * TP + 31]);
   __syncwarp();
-  // a halo pixel's contribution goes into one value per border pixel (8-connected: the three beside it)
-  if (CONN8) {
-    auto up1 = [](T v, T first) { const T n = (T)__shfl_up_sync(0xffffffffu, (unsigned)v, 1); return (threadIdx.x & 31) == 0 ? first : n; };
-    auto dn1 = [](T v, T last) { const T n = (T)__shfl_down_sync(0xffffffffu, (unsigned)v, 1); return (threadIdx.x & 31) == 31 ? last : n; };
-    const T bl = (T)__shfl_sync(0xffffffffu, (unsigned)c_bot, 0), tr = (T)__shfl_sync(0xffffffffu, (unsigned)c_top, 31);
-    const T t3 = OT::apply(h_top, OT::apply(up1(h_top, c_top), dn1(h_top, c_top)));
-    const T b3 = OT::apply(h_bot, OT::apply(up1(h_bot, c_bot), dn1(h_bot, c_bot)));
-    const T l3 = OT::apply(h_l, OT::apply(up1(h_l, c_top), dn1(h_l, bl)));
-    const T r3 = OT::apply(h_r, OT::apply(up1(h_r, tr), dn1(h_r, c_bot)));
-    h_top = t3; h_bot = b3; h_l = l3; h_r = r3;
-  }
+  if (CONN8) fold_halo<T, SUP>(h_top, h_bot, h_l, h_r, c_top, c_bot);
   const uint32_t tb = pk2(h_top, h_bot), lr = pk2(h_l, h_r);
 
-  auto OS = [](uint32_t a, uint32_t b) { return SUP ? u16x2_max(a, b) : u16x2_min(a, b); };  // propagation
-  auto OC = [](uint32_t a, uint32_t b) { return SUP ? u16x2_min(a, b) : u16x2_max(a, b); };  // clip by the mask
-  auto nbrow = [&](uint32_t x) -> uint32_t {
-    if (CONN8) {
-      const uint32_t a = __shfl_up_sync(0xffffffffu, x, 1), b = __shfl_down_sync(0xffffffffu, x, 1);
-      return OS(x, OS(a, b));
-    }
-    return x;
-  };
-  const uint32_t *MAs = s.ma + lane, *MBs = s.mb + lane;
-  bool converged = false, changed = false;
   uint32_t end_lr = init_lr;
-  for (int sweep = 0; sweep < P.max_sweeps; ++sweep) {
-    uint32_t ch = 0;
-    // vertical: pair k from pair k - 1 (k = 0: the halo rows), then pair 15 from itself swapped and pair q
-    // from pair q + 1
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const uint32_t nb = k == 0 ? tb : nbrow(V[k - 1]);  // the halo rows are already 3-wide
-      const uint32_t nv = OC(OS(V[k], nb), lds_u32(MAs + k * kRP));
-      ch |= nv ^ V[k];
-      V[k] = nv;
-    }
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int q = 15 - k;
-      const uint32_t nb = nbrow(k == 0 ? swap2(V[15]) : V[q + 1]);
-      const uint32_t nv = OC(OS(V[q], nb), lds_u32(MAs + q * kRP));
-      ch |= nv ^ V[q];
-      V[q] = nv;
-    }
-    // to lane = row
-#pragma unroll
-    for (int p = 0; p < 16; ++p) {
-      s.val[p * TP + lane] = (T)V[p];
-      s.val[(31 - p) * TP + lane] = (T)(V[p] >> 16);
-    }
-    __syncwarp();
-    uint32_t Q[16];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) Q[c] = pk2(s.val[lane * TP + c], s.val[lane * TP + 31 - c]);
-    __syncwarp();
-    // horizontal, the same pairing
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const uint32_t nb = k == 0 ? lr : Q[k - 1];
-      const uint32_t nv = OC(OS(Q[k], nb), lds_u32(MBs + k * kRP));
-      ch |= nv ^ Q[k];
-      Q[k] = nv;
-    }
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int q = 15 - k;
-      const uint32_t nb = k == 0 ? swap2(Q[15]) : Q[q + 1];
-      const uint32_t nv = OC(OS(Q[q], nb), lds_u32(MBs + q * kRP));
-      ch |= nv ^ Q[q];
-      Q[q] = nv;
-    }
-    end_lr = Q[0];
-    if (!__any_sync(0xffffffffu, ch != 0)) {
-      converged = true;  // nothing moved: V still holds the values
-      break;
-    }
-    changed = true;
-    // back to lane = column
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      s.val[lane * TP + c] = (T)Q[c];
-      s.val[lane * TP + 31 - c] = (T)(Q[c] >> 16);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int p = 0; p < 16; ++p) V[p] = pk2(s.val[p * TP + lane], s.val[(31 - p) * TP + lane]);
-    __syncwarp();
-  }
+  bool changed = false;
+  const bool converged = packed_sweeps<T, SUP, CONN8>(V, s, tb, lr, P.max_sweeps, end_lr, changed);
 
   const uint32_t d_tb = V[0] ^ init_tb, d_lr = end_lr ^ init_lr;
   const unsigned bN = __ballot_sync(0xffffffffu, (d_tb & 0xffffu) != 0u), bS = __ballot_sync(0xffffffffu, (d_tb >> 16) != 0u);
@@ -1374,6 +1403,279 @@ __global__ void __launch_bounds__(kRegWarps * 32, sizeof(T) <= 2 ? 5 : 4) k_reco
   recon_epilogue<T, SUP>(P, begin);
 }
 
+// ------------------------------------------------------------------ resident tiles
+// Images of 1- or 2-byte pixels whose tiles all fit on the GPU at once (32 warps per SM: 4864 tiles of 32 x 32,
+// 5 Mpixel) keep every tile in one warp from start to end: the values in registers, the mask in shared memory.
+// No tile is staged again, nothing is queued: a visit reads its neighbours' border pixels, sweeps, publishes its
+// own changed borders (32 contiguous pixels each) and marks the neighbours beside them; a warp with nothing to do
+// polls its tile's state word.  A value crosses a tile in the time of one border load, the sweeps, one fence and
+// one atomic, where the worklist also pops, stages, writes back and queues.
+//
+// State of a tile: RS_IDLE, RS_RUNNING (its warp is visiting), RS_DIRTY (a border beside it changed since the
+// visit read its halo).  `pending` counts the tiles that are not idle.  A warp adds the neighbours it may wake
+// before it marks them and takes off the ones that were awake already, and itself when it falls idle,
+// afterwards: `pending` never reads zero early, and the warp that brings it to zero ends the kernel.
+// Bound: the chain of dependent visits (border load, two sweep sets, fence, atomic: about 4 us a hop).  Kernel
+// alone, by ncu: binary h-maxima 2048^2 u8 110 -> 71 us, one half of the leveling of 1537 x 1805 u16 250 -> 78 us;
+// calls 131 -> 93 and 555 -> 192 us.  One to 64 sweep sets per visit: 93-101 us, two kept.
+enum : unsigned { RS_IDLE = 0, RS_RUNNING = 1, RS_DIRTY = 2 };
+static constexpr int kResidentWarps = 32;
+
+struct ResCtl {  // in the work area, cleared before the launch
+  int pending, pad0[31];
+  int done, pad1[31];
+};
+static_assert(sizeof(ResCtl) == 256, "ResCtl layout");
+
+template <typename T> struct ResTiles {
+  ResCtl *ctl;
+  unsigned *state;  // ntiles
+  T *border;        // ntiles x 4 x 32 pixels: rows top and bottom, columns left and right
+};
+
+__device__ __forceinline__ unsigned exch_acquire(unsigned *p, unsigned v) {
+  unsigned old;
+  asm volatile("atom.acquire.gpu.global.exch.b32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
+}
+
+template <typename T, bool SUP, bool CONN8>
+__global__ void __launch_bounds__(kResidentWarps * 32, 1) k_reconstruct_resident(const __grid_constant__ RParams<T> P,
+                                                                                const ResTiles<T> rt) {
+  static_assert(sizeof(T) <= 2, "packed tiles");
+  using OT = Op<T, SUP>;
+  constexpr int TP = PackedCore<T>::TP;
+  constexpr int LR = TileRows<T, true>::LR, RI = TileRows<T, true>::RI, PASSES = TileRows<T, true>::PASSES;
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  PackedCore<T> &s = reinterpret_cast<PackedCore<T> *>(s_dyn)[warp];
+  RCtl *ctl = P.ctl;
+  const T NEU = OT::neutral();
+  // tiles are dealt over the SMs, so that a front of active tiles is spread over all of them
+  const int t = (int)(blockIdx.x + gridDim.x * (unsigned)warp);
+  const bool have = t < P.ntiles;
+  int tl = 0;
+  const RImg &im = image_of(P, have ? t : 0, tl);
+  const int tx = tl % im.tiles_x, ty = tl / im.tiles_x;
+  const int64_t y0 = (int64_t)ty * 32, x0 = (int64_t)tx * 32;
+  const int rows = (int)min((int64_t)32, im.H - y0), cols = (int)min((int64_t)32, im.W - x0);
+  T *mine = rt.border + (size_t)t * 128;
+  uint32_t V[16], pub_lr = 0;
+
+  if (have) {
+    // the reference (or mask), then the marker, through s.val into registers: effective mask and initial value
+    auto stage = [&](const void *img) {
+      const TileRows<T, false> r(img, im, y0, x0, rows);
+#pragma unroll
+      for (int k0 = 0; k0 < PASSES; k0 += 4) {
+        uint32_t w[4][3];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r.load(k0 + k, (k0 + k) * RI + lane / LR < rows, im, w[k]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint2 v = r.pixels(k0 + k, w[k]);
+          uint32_t *d = reinterpret_cast<uint32_t *>(s.val + ((k0 + k) * RI + lane / LR) * TP) + 2 * (lane % LR);
+          d[0] = v.x;
+          d[1] = v.y;
+        }
+      }
+      __syncwarp();
+    };
+    uint32_t M[16];
+    stage(im.mask);
+#pragma unroll
+    for (int p = 0; p < 16; ++p) M[p] = pk2(s.val[p * TP + lane], s.val[(31 - p) * TP + lane]);
+    if (P.init != INIT_SAT_CONST) {
+      __syncwarp();
+      stage(im.marker);
+    }
+    auto pixel = [&](int r, uint32_t ref, T &m, T &v) {  // pixel (r, lane)
+      m = v = NEU;
+      if (r < rows && lane < cols) combine_init<T, SUP>(P, (T)ref, s.val[r * TP + lane], m, v);
+    };
+#pragma unroll
+    for (int p = 0; p < 16; ++p) {
+      T m0, m1, v0, v1;
+      pixel(p, M[p], m0, v0);
+      pixel(31 - p, M[p] >> 16, m1, v1);
+      M[p] = pk2(m0, m1);
+      V[p] = pk2(v0, v1);
+    }
+    // both by rows, for the column pairs
+    auto by_rows = [&](const uint32_t (&x)[16]) {
+      __syncwarp();
+#pragma unroll
+      for (int p = 0; p < 16; ++p) {
+        s.val[p * TP + lane] = (T)x[p];
+        s.val[(31 - p) * TP + lane] = (T)(x[p] >> 16);
+      }
+      __syncwarp();
+    };
+    by_rows(M);
+#pragma unroll
+    for (int p = 0; p < 16; ++p) {
+      s.ma[p * kRP + lane] = M[p];
+      s.mb[p * kRP + lane] = pk2(s.val[lane * TP + p], s.val[lane * TP + 31 - p]);
+    }
+    by_rows(V);
+    pub_lr = pk2(s.val[lane * TP], s.val[lane * TP + 31]);
+    st_cg(mine + lane, (T)V[0]);
+    st_cg(mine + 32 + lane, (T)(V[0] >> 16));
+    st_cg(mine + 64 + lane, (T)pub_lr);
+    st_cg(mine + 96 + lane, (T)(pub_lr >> 16));
+    if (lane == 0) rt.state[t] = RS_RUNNING;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    rt.ctl->pending = P.ntiles;
+    g_recon_rounds = 0;
+  }
+  if (!grid_barrier(ctl, P.wait_ns)) return;
+  if (!have) return;
+
+  // lane d < 8 looks after the neighbour in direction d = N S W E NW NE SW SE (B_x = 1 << d)
+  int nb = -1;
+  if (lane < (CONN8 ? 8 : 4)) {
+    const int dx = lane < 2 ? 0 : ((lane & 1) ? 1 : -1);
+    const int dy = lane < 2 ? (lane ? 1 : -1) : lane < 4 ? 0 : (lane < 6 ? -1 : 1);
+    const int nx = tx + dx, ny = ty + dy;
+    if (nx >= 0 && ny >= 0 && nx < im.tiles_x && ny < im.tiles_y) nb = t + dy * im.tiles_x + dx;
+  }
+  const bool up = ty > 0, down = ty + 1 < im.tiles_y, west = tx > 0, east = tx + 1 < im.tiles_x;
+  int visits = 0;
+  for (;;) {
+    // ---- visit: the halo from the neighbours' borders
+    if (++visits > P.max_rounds) {
+      if (lane == 0) set_status(ctl, PG_ERR_NOT_CONVERGED);
+      return;
+    }
+    T h_top = NEU, h_bot = NEU, h_l = NEU, h_r = NEU, c_top = NEU, c_bot = NEU;
+    {
+      const T *b = rt.border + (size_t)t * 128 + lane;
+      const int down_row = im.tiles_x * 128;
+      if (up) h_top = ld_cg(b - down_row + 32);
+      if (down) h_bot = ld_cg(b + down_row);
+      if (west) h_l = ld_cg(b - 128 + 96);
+      if (east) h_r = ld_cg(b + 128 + 64);
+      if (CONN8 && ((lane == 0 && west) || (lane == 31 && east))) {
+        const T *c = lane == 0 ? b - 128 + 31 : b + 128 - 31;  // the last / first pixel of that neighbour's rows
+        if (up) c_top = ld_cg(c - down_row + 32);
+        if (down) c_bot = ld_cg(c + down_row);
+      }
+    }
+    if (CONN8) fold_halo<T, SUP>(h_top, h_bot, h_l, h_r, c_top, c_bot);
+    const uint32_t init_tb = V[0];
+    uint32_t end_lr = pub_lr;
+    bool changed = false;
+    const bool converged = packed_sweeps<T, SUP, CONN8>(V, s, pk2(h_top, h_bot), pk2(h_l, h_r), P.max_sweeps, end_lr, changed);
+
+    // ---- the borders that changed, and the neighbours beside them
+    const uint32_t d_tb = V[0] ^ init_tb, d_lr = end_lr ^ pub_lr;
+    const unsigned bN = __ballot_sync(0xffffffffu, (d_tb & 0xffffu) != 0u), bS = __ballot_sync(0xffffffffu, (d_tb >> 16) != 0u);
+    const unsigned bW = __ballot_sync(0xffffffffu, (d_lr & 0xffffu) != 0u), bE = __ballot_sync(0xffffffffu, (d_lr >> 16) != 0u);
+    pub_lr = end_lr;
+    if (bN) st_cg(mine + lane, (T)V[0]);
+    if (bS) st_cg(mine + 32 + lane, (T)(V[0] >> 16));
+    if (bW) st_cg(mine + 64 + lane, (T)pub_lr);
+    if (bE) st_cg(mine + 96 + lane, (T)(pub_lr >> 16));
+    bool wake = false;
+    if (nb >= 0) {
+      const unsigned of = lane == 0 ? bN : lane == 1 ? bS : lane == 2 ? bW : lane == 3 ? bE
+                          : lane == 4 ? (bN & 1u) : lane == 5 ? (bN >> 31) : lane == 6 ? (bS & 1u) : (bS >> 31);
+      wake = of != 0u;
+    }
+    const int n_wake = __popc(__ballot_sync(0xffffffffu, wake));
+    int off = 0;  // tiles to take off `pending` again
+    if (n_wake) {
+      if (lane == 0) atomicAdd(&rt.ctl->pending, n_wake);
+      __threadfence();  // the borders and the count before the marks
+      __syncwarp();
+      const bool awake = wake && atomicExch(rt.state + nb, RS_DIRTY) != RS_IDLE;
+      off = __popc(__ballot_sync(0xffffffffu, awake));
+    }
+    // ---- back to idle, or on with another visit
+    unsigned again = 1;
+    if (lane == 0) {
+      if (converged && atomicCAS(rt.state + t, RS_RUNNING, RS_IDLE) == RS_RUNNING) {
+        again = 0;
+        ++off;
+      }
+      if (off && atomicSub(&rt.ctl->pending, off) == off) *((volatile int *)&rt.ctl->done) = 1;
+    }
+    again = __shfl_sync(0xffffffffu, again, 0);
+    int stop = 0;
+    if (lane == 0) {
+      if (!again) {
+        const unsigned long long t0 = global_ns();
+        for (unsigned polls = 0;; ++polls) {
+          if (*((volatile unsigned *)(rt.state + t)) == RS_DIRTY) break;
+          if (polls % 8 == 7) {
+            if (*((volatile int *)&rt.ctl->done)) { stop = 1; break; }
+            if (*((volatile int *)&ctl->status)) { stop = 2; break; }
+            if (wait_expired(ctl, t0, P.wait_ns)) { stop = 2; break; }
+          }
+          __nanosleep(polls < 16 ? 20 : 100);
+        }
+      } else if (*((volatile int *)&ctl->status)) {
+        stop = 2;
+      }
+      if (!stop) exch_acquire(rt.state + t, RS_RUNNING);  // before the halo is read: what changes later marks again
+    }
+    stop = __shfl_sync(0xffffffffu, stop, 0);
+    if (stop == 2) return;
+    if (stop == 1) break;
+  }
+  if (lane == 0) atomicMax(&g_recon_rounds, visits);
+
+  // ---- result: the values by rows in shared memory, then the epilogue's function of them and the reference
+  __syncwarp();
+#pragma unroll
+  for (int p = 0; p < 16; ++p) {
+    s.val[p * TP + lane] = (T)V[p];
+    s.val[(31 - p) * TP + lane] = (T)(V[p] >> 16);
+  }
+  __syncwarp();
+  if (P.epi == EPI_BINARY_SUP) {  // the mask here is the reference itself
+    uint8_t *o = static_cast<uint8_t *>(im.out) + y0 * im.W + x0 + lane;
+    if (lane < cols)
+#pragma unroll 8
+      for (int r = 0; r < rows; ++r) {
+        const T ref = (T)(r < 16 ? s.ma[r * kRP + lane] : s.ma[(31 - r) * kRP + lane] >> 16);
+        o[r * im.W] = epi_binary<T, SUP>(ref, s.val[r * TP + lane]);
+      }
+    return;
+  }
+  const TileRows<T, true> ro(im.out, im, y0, x0, rows);
+  if (P.epi == EPI_CLIP_REF) {
+    const TileRows<T, false> rr(im.mask, im, y0, x0, rows);
+#pragma unroll
+    for (int k0 = 0; k0 < PASSES; k0 += 4) {
+      uint32_t w[4][3];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) rr.load(k0 + k, (k0 + k) * RI + lane / LR < rows, im, w[k]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint2 v = rr.pixels(k0 + k, w[k]);
+        uint32_t *d = reinterpret_cast<uint32_t *>(s.val + ((k0 + k) * RI + lane / LR) * TP) + 2 * (lane % LR);
+        d[0] = wop<T, !SUP>(d[0], v.x);
+        d[1] = wop<T, !SUP>(d[1], v.y);
+      }
+    }
+    __syncwarp();
+  }
+  if (ro.pairs && cols == 32) {
+#pragma unroll
+    for (int k = 0; k < PASSES; ++k) {
+      const int row = k * RI + lane / LR;
+      const uint32_t *d = reinterpret_cast<const uint32_t *>(s.val + row * TP) + 2 * (lane % LR);
+      if (row < rows) *reinterpret_cast<uint2 *>(ro.a + k * ro.pitch) = make_uint2(d[0], d[1]);
+    }
+  } else if (lane < cols) {
+    T *o = static_cast<T *>(im.out) + y0 * im.W + x0 + lane;
+#pragma unroll 8
+    for (int r = 0; r < rows; ++r) o[r * im.W] = s.val[r * TP + lane];
+  }
+}
+
 // ------------------------------------------------------------------ host side
 // Scratch work area of one launch: control block (256 B) | worklist counters (512 B) | per-tile
 // words: the double-buffered flags of the round kernel, or the tile states and the ring of the
@@ -1446,6 +1748,50 @@ static pg_status launch_recon(RParams<T> &P, char *work, cudaStream_t s, int *gr
   return PG_OK;
 }
 
+// Whether the resident kernel holds this many tiles, and its launch.  `work` is a cleared work area of
+// resident_bytes().
+static size_t resident_bytes(int64_t ntiles, size_t elem_bytes) {
+  return 256 + sizeof(ResCtl) + (4 * (size_t)ntiles + 255) / 256 * 256 + 128 * (size_t)ntiles * elem_bytes;
+}
+static bool resident_fits(int64_t ntiles) { return ntiles <= (int64_t)kResidentWarps * num_sms(); }
+
+template <typename T, bool SUP, bool CONN8>
+static pg_status launch_resident(RParams<T> &P, char *work, cudaStream_t s) {
+  static_assert(sizeof(PackedCore<T>) * kResidentWarps <= 227 * 1024, "a CTA's tiles fit in shared memory");
+  P.ctl = reinterpret_cast<RCtl *>(work);
+  P.max_rounds = max_rounds_for(P.ntiles);
+  P.wait_ns = g_dbg_wait_ns.load();
+  ResTiles<T> rt{};
+  rt.ctl = reinterpret_cast<ResCtl *>(work + 256);
+  rt.state = reinterpret_cast<unsigned *>(work + 256 + sizeof(ResCtl));
+  rt.border = reinterpret_cast<T *>(work + 256 + sizeof(ResCtl) + (4 * (size_t)P.ntiles + 255) / 256 * 256);
+  const int grid = std::min(num_sms(), P.ntiles);
+  const int warps = (int)ceil_div(P.ntiles, grid);
+  const size_t smem = sizeof(PackedCore<T>) * (size_t)warps;
+  static std::atomic<uint64_t> attr_devices{0};  // the opt-in shared-memory size, once per device
+  int dev = 0;
+  PG_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
+  const uint64_t bit = 1ull << (dev & 63);
+  if (!(attr_devices.load() & bit)) {
+    PG_CUDA_TRY(cudaFuncSetAttribute(k_reconstruct_resident<T, SUP, CONN8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(sizeof(PackedCore<T>) * kResidentWarps)),
+                "resident reconstruction smem attribute");
+    attr_devices.fetch_or(bit);
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)warps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  PG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_reconstruct_resident<T, SUP, CONN8>, P, rt), "cooperative reconstruction launch");
+  return PG_OK;
+}
+
 template <typename T, bool SUP, bool CONN8>
 static pg_status run_t(std::vector<RImg> &imgs, const ReconRequest &rq, bool binary, cudaStream_t s) {
   // register tiles (32x32, a warp each) up to 4-byte pixels, shared-memory tiles for 8-byte ones
@@ -1461,6 +1807,24 @@ static pg_status run_t(std::vector<RImg> &imgs, const ReconRequest &rq, bool bin
   }
   if (ntiles == 0) return PG_OK;
   const int nimg = (int)imgs.size();
+  if constexpr (sizeof(T) <= 2) {
+    if (nimg == 1 && resident_fits(ntiles)) {
+      Scratch work;
+      PG_TRY(work.alloc(resident_bytes(ntiles, sizeof(T)), s));
+      // control words and states; the borders are written before they are read
+      PG_CUDA_TRY(cudaMemsetAsync(work.ptr, 0, 256 + sizeof(ResCtl) + 4 * (size_t)ntiles, s), "clear reconstruction work area");
+      RParams<T> P{};
+      P.single = imgs[0];
+      P.nimg = 1;
+      P.ntiles = ntiles;
+      P.init = rq.init;
+      P.mask_mode = rq.mask_mode;
+      P.epi = rq.epi;
+      P.h = scalar_as<T>(rq.h);
+      P.max_sweeps = kVisitSweeps;
+      return launch_resident<T, SUP, CONN8>(P, work.as<char>(), s);
+    }
+  }
   // scratch: work area | image table | reconstruction buffers (binary mode)
   const size_t off_tab = work_bytes(ntiles);
   const size_t off_rec = off_tab + ((sizeof(RImg) * (size_t)(nimg > 1 ? nimg : 0) + 255) / 256) * 256;
