@@ -388,6 +388,232 @@ __global__ void __launch_bounds__(AT_THREADS) k_flat_bwd_arg(const unsigned char
   }
 }
 
+// ------------------------------------------------------------------ rows streamed through registers
+// The saved-arg pair for rows of whole 16-byte vectors.  A half warp owns a segment of 64 columns (a lane four)
+// and walks down a strip of rows; the columns beside a lane's come from its neighbours by shuffles, those beside
+// the segment from loads of its first and last lane.  No shared memory and no barrier: the loads of 2R + 1 rows
+// are issued together and every warp streams on its own.
+//
+// Forward: a row's best value and first best column per pixel, then the same down the columns over a ring of
+// 2R + 1 rows in registers.  An arg is found as "the last candidate, replaced by every earlier one whose value
+// equals the best", with the replacement as a multiply-add by the 0 / 1 of the comparison: min, max, compare and
+// select all issue on the half-rate ALU pipe, which the selects alone would fill.
+// Backward: code(p) names the one input pixel output p routes to, so row p.y adds to the 2R + 1 input rows
+// around it: accumulators in a ring of registers.  Two candidates are tested in one comparison of 16-bit pairs
+// (a code in both bytes of a half: codes up to 48 are distinct numbers, 255 outside the image is a NaN and
+// equals nothing), each of the two predicates guards one addition.  Rows, then columns in ascending order: the
+// sums are in raster order of the outputs.
+// [64, 32, 256, 256] f32, 5x5 window: forward 375 us (shared-memory tiles above) -> 254, backward 448 -> 332; floor
+// 178 us each (9 bytes a pixel).  3x3: 298 -> 219 and 305 -> 196; 7x7: 481 -> 323 and 764 -> 690.  The backward
+// is bound by the ALU pipe (64 % busy: one comparison per candidate, 25 a pixel), the forward by the ALU (55 %)
+// and by load latency at 24 warps per SM.
+static constexpr int AS_LANES = 16, AS_COLS = 4 * AS_LANES, AS_THREADS = 128;
+
+struct StripGeom {
+  int H, W, strip;      // rows, columns, rows of a strip
+  int segs, strips;     // segments per row, strips per plane
+  int64_t units;        // planes * strips * segs
+};
+
+__device__ __forceinline__ float eq01(float a, float b) {  // 1 where a == b, else 0
+  float r;
+  asm("set.eq.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+template <bool SUP, int R>
+__global__ void __launch_bounds__(AS_THREADS) k_flat_fwd_arg_strip(const float *__restrict__ x, float *__restrict__ y,
+                                                                   unsigned char *__restrict__ code, const StripGeom g) {
+  constexpr int WX = 2 * R + 1, NE = 4 + 2 * R;
+  const int64_t u = ((int64_t)blockIdx.x * AS_THREADS + threadIdx.x) / AS_LANES;
+  const int l = threadIdx.x % AS_LANES;
+  const bool live = u < g.units;
+  const int64_t uu = live ? u : g.units - 1;
+  const int seg = (int)(uu % g.segs), strip = (int)(uu / g.segs % g.strips);
+  const int64_t plane = uu / g.segs / g.strips * ((int64_t)g.H * g.W);
+  const int x0 = seg * AS_COLS + 4 * l, y0 = strip * g.strip, y1 = min(y0 + g.strip, g.H);
+  const bool in = x0 < g.W;
+  // the first lane brings the R columns left of the segment, the last one those on its right
+  const int xe = l == 0 ? x0 - R : x0 + 4;
+  const bool edge = l == 0 || l == AS_LANES - 1;
+  const float *xp = x + plane;
+  float rv[WX][4], rc[WX][4];  // ring: row-best values and their columns in the window
+#pragma unroll
+  for (int i = 0; i < WX; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) rv[i][j] = rc[i][j] = 0.f;
+  // row r of the walk is image row y0 - R + r; output row r - 2R is formed with it
+  const int n = y1 - y0 + 2 * R;
+  for (int r0 = 0; r0 < g.strip + 2 * R; r0 += WX) {
+    float4 v[WX];
+    float ex[WX][R];
+#pragma unroll
+    for (int i = 0; i < WX; ++i) {
+      const int yy = y0 - R + r0 + i;
+      const bool row = r0 + i < n && yy >= 0 && yy < g.H;
+      const float *p = xp + (int64_t)yy * g.W;
+      const float o = outside<SUP>();
+      v[i] = row && in ? __ldg(reinterpret_cast<const float4 *>(p + x0)) : make_float4(o, o, o, o);
+#pragma unroll
+      for (int k = 0; k < R; ++k) ex[i][k] = row && edge && xe + k >= 0 && xe + k < g.W ? __ldg(p + xe + k) : o;
+    }
+#pragma unroll
+    for (int i = 0; i < WX; ++i) {
+      float e[NE];
+      const float own[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) e[R + j] = own[j];
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        const float a = __shfl_up_sync(0xffffffffu, own[4 - R + k], 1, AS_LANES);
+        const float b = __shfl_down_sync(0xffffffffu, own[k], 1, AS_LANES);
+        e[k] = l == 0 ? ex[i][k] : a;
+        e[R + 4 + k] = l == AS_LANES - 1 ? ex[i][k] : b;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float b = e[j];
+#pragma unroll
+        for (int d = 1; d <= 2 * R; ++d) b = best_of<SUP>(b, e[j + d]);
+        float a = 2.f * R;
+#pragma unroll
+        for (int d = 2 * R - 1; d >= 0; --d) a = fmaf(eq01(e[j + d], b), (float)d - a, a);
+        rv[i][j] = b;
+        rc[i][j] = a;
+      }
+      const int out = r0 + i - 2 * R;  // output row of the strip; its window's row d is ring slot (i + 1 + d) % WX
+      if (out < 0 || y0 + out >= y1) continue;
+      float best[4], cd[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float b = rv[(i + 1) % WX][j];
+#pragma unroll
+        for (int d = 1; d <= 2 * R; ++d) b = best_of<SUP>(b, rv[(i + 1 + d) % WX][j]);
+        float c = rc[i][j] + (float)(2 * R * WX);
+#pragma unroll
+        for (int d = 2 * R - 1; d >= 0; --d)
+          c = fmaf(eq01(rv[(i + 1 + d) % WX][j], b), rc[(i + 1 + d) % WX][j] + (float)(d * WX) - c, c);
+        best[j] = b;
+        cd[j] = c + 8388608.f;  // 2^23: the code is the low byte of the sum
+      }
+      if (live && in) {
+        const int64_t o = plane + (int64_t)(y0 + out) * g.W + x0;
+        __stcs(reinterpret_cast<float4 *>(y + o), make_float4(best[0], best[1], best[2], best[3]));
+        const uint32_t lo = __byte_perm(__float_as_uint(cd[0]), __float_as_uint(cd[1]), 0x0040);
+        const uint32_t hi = __byte_perm(__float_as_uint(cd[2]), __float_as_uint(cd[3]), 0x0040);
+        __stcs(reinterpret_cast<unsigned int *>(code + o), __byte_perm(lo, hi, 0x5410));
+      }
+    }
+  }
+}
+
+// acc0 += g0 where the low half of `pair` equals that of `want`, acc1 += g1 where the high half does
+__device__ __forceinline__ void add_if(float &acc0, float &acc1, uint32_t pair, uint32_t want, float g0, float g1) {
+  asm("{\n .reg .pred p, q;\n setp.eq.f16x2 p|q, %2, %3;\n @p add.f32 %0, %0, %4;\n @q add.f32 %1, %1, %5;\n}"
+      : "+f"(acc0), "+f"(acc1)
+      : "r"(pair), "r"(want), "f"(g0), "f"(g1));
+}
+
+template <int R>
+__global__ void __launch_bounds__(AS_THREADS) k_flat_bwd_arg_strip(const unsigned char *__restrict__ code,
+                                                                   const float *__restrict__ gy, float *__restrict__ gx,
+                                                                   const StripGeom g) {
+  constexpr int WX = 2 * R + 1, NE = 4 + 2 * R;
+  const int64_t u = ((int64_t)blockIdx.x * AS_THREADS + threadIdx.x) / AS_LANES;
+  const int l = threadIdx.x % AS_LANES;
+  const bool live = u < g.units;
+  const int64_t uu = live ? u : g.units - 1;
+  const int seg = (int)(uu % g.segs), strip = (int)(uu / g.segs % g.strips);
+  const int64_t plane = uu / g.segs / g.strips * ((int64_t)g.H * g.W);
+  const int x0 = seg * AS_COLS + 4 * l, y0 = strip * g.strip, y1 = min(y0 + g.strip, g.H);
+  const bool in = x0 < g.W;
+  const int xe = l == 0 ? x0 - 4 : x0 + 4;  // the vector beside the segment
+  const bool edge = (l == 0 || l == AS_LANES - 1) && xe >= 0 && xe < g.W;
+  const float *gp = gy + plane;
+  const unsigned char *cp = code + plane;
+  float acc[WX][4];  // ring: input row y0 - 2R + r of the walk's row r sits in slot r % WX
+#pragma unroll
+  for (int i = 0; i < WX; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  // row r of the walk is output row y0 - R + r; it adds to input rows y0 - 2R + r .. y0 + r
+  const int n = y1 - y0 + 2 * R;
+  for (int r0 = 0; r0 < g.strip + 2 * R; r0 += WX) {
+    float4 v[WX];
+    uint32_t c[WX], ce[WX];
+    float ex[WX][R];
+#pragma unroll
+    for (int i = 0; i < WX; ++i) {
+      const int yy = y0 - R + r0 + i;
+      const bool row = r0 + i < n && yy >= 0 && yy < g.H;
+      const int64_t o = (int64_t)yy * g.W;
+      v[i] = row && in ? __ldg(reinterpret_cast<const float4 *>(gp + o + x0)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      c[i] = row && in ? __ldg(reinterpret_cast<const unsigned int *>(cp + o + x0)) : 0xffffffffu;
+      ce[i] = row && edge ? __ldg(reinterpret_cast<const unsigned int *>(cp + o + xe)) : 0xffffffffu;
+#pragma unroll
+      for (int k = 0; k < R; ++k) ex[i][k] = row && edge ? __ldg(gp + o + (l == 0 ? x0 - R : x0 + 4) + k) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < WX; ++i) {
+      const float own[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+      float e[NE];  // upstream gradients of columns x0 - R .. x0 + 3 + R
+#pragma unroll
+      for (int j = 0; j < 4; ++j) e[R + j] = own[j];
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        const float a = __shfl_up_sync(0xffffffffu, own[4 - R + k], 1, AS_LANES);
+        const float b = __shfl_down_sync(0xffffffffu, own[k], 1, AS_LANES);
+        e[k] = l == 0 ? ex[i][k] : a;
+        e[R + 4 + k] = l == AS_LANES - 1 ? ex[i][k] : b;
+      }
+      const uint32_t cl = __shfl_up_sync(0xffffffffu, c[i], 1, AS_LANES), cr = __shfl_down_sync(0xffffffffu, c[i], 1, AS_LANES);
+      const uint32_t w[3] = {l == 0 ? ce[i] : cl, c[i], l == AS_LANES - 1 ? ce[i] : cr};
+      uint32_t pr[NE - 1];  // codes of columns k and k + 1 (from x0 - R), each in both bytes of its half
+#pragma unroll
+      for (int k = 0; k < NE - 1; ++k) {
+        const int p = 4 - R + k, q = p % 4;  // byte of the first in w
+        pr[k] = __byte_perm(w[p / 4], p / 4 < 2 ? w[p / 4 + 1] : 0u, q | (q << 4) | ((q + 1) << 8) | ((q + 1) << 12));
+      }
+      // input row t of the 2R + 1 (arg row t of the window): slot (i + t) % WX; columns in ascending order
+#pragma unroll
+      for (int t = 0; t < WX; ++t)
+#pragma unroll
+        for (int b = 0; b < WX; ++b) {
+          const uint32_t want = 0x01010101u * (uint32_t)(t * WX + 2 * R - b);
+#pragma unroll
+          for (int j = 0; j < 4; j += 2)
+            add_if(acc[(i + t) % WX][j], acc[(i + t) % WX][j + 1], pr[j + b], want, e[j + b], e[j + b + 1]);
+        }
+      // the first of those input rows has all its outputs now
+      const int out = r0 + i - 2 * R;
+      if (out >= 0 && y0 + out < y1 && live && in)
+        __stcs(reinterpret_cast<float4 *>(gx + plane + (int64_t)(y0 + out) * g.W + x0),
+               make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    }
+  }
+}
+
+// Whether the strip kernels take these planes, and their geometry.
+static bool strip_geom(const void *a, const void *b, const void *code, int64_t planes, int64_t h, int64_t w, StripGeom &g) {
+  if (w % 4 != 0 || (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % 16 != 0 ||
+      reinterpret_cast<uintptr_t>(code) % 4 != 0)
+    return false;
+  g.H = (int)h;
+  g.W = (int)w;
+  g.segs = (int)ceil_div(w, AS_COLS);
+  // strips of 64 rows, shorter where the planes would not give every SM 24 warps (675 planes of 80 x 240, 5x5: 16
+  // warps 36 + 50 us, 24 35 + 52, 64 41 + 61)
+  g.strip = 64;
+  auto units = [&] { return planes * ceil_div(h, g.strip) * g.segs; };
+  while (g.strip > 8 && units() < (int64_t)num_sms() * 48) g.strip /= 2;
+  g.strips = (int)ceil_div(h, g.strip);
+  g.strip = (int)ceil_div(h, g.strips);  // evenly
+  g.units = planes * g.strips * g.segs;
+  return ceil_div(g.units * AS_LANES, AS_THREADS) <= INT32_MAX;
+}
+
 template <bool SUP>
 static bool flat_fwd_fixed(const float *x, float *y, int64_t planes, int64_t h, int64_t w, int ry, int rx, cudaStream_t s) {
   if (ry != rx || ry < 1 || ry > 3 || planes > 65535) return false;
@@ -661,6 +887,20 @@ pg_status launch_flat2d_arg(const float *x, float *y, unsigned char *code, int64
   if (planes * h * w == 0) return PG_OK;
   if (h > (1 << 30) || w > (1 << 30) || ceil_div(h, AT_H) > 65535 || planes > 65535)
     return fail(PG_ERR_INVALID_ARGUMENT, "plane too large");
+  StripGeom g;
+  if (strip_geom(x, y, code, planes, h, w, g)) {
+    const unsigned ctas = (unsigned)ceil_div(g.units * AS_LANES, AS_THREADS);
+    if (dilate) {
+      if (r == 1) k_flat_fwd_arg_strip<true, 1><<<ctas, AS_THREADS, 0, s>>>(x, y, code, g);
+      else if (r == 2) k_flat_fwd_arg_strip<true, 2><<<ctas, AS_THREADS, 0, s>>>(x, y, code, g);
+      else k_flat_fwd_arg_strip<true, 3><<<ctas, AS_THREADS, 0, s>>>(x, y, code, g);
+    } else {
+      if (r == 1) k_flat_fwd_arg_strip<false, 1><<<ctas, AS_THREADS, 0, s>>>(x, y, code, g);
+      else if (r == 2) k_flat_fwd_arg_strip<false, 2><<<ctas, AS_THREADS, 0, s>>>(x, y, code, g);
+      else k_flat_fwd_arg_strip<false, 3><<<ctas, AS_THREADS, 0, s>>>(x, y, code, g);
+    }
+    return cuda_status(cudaGetLastError(), "flat morphology forward (saved arg) launch");
+  }
   const dim3 grid((unsigned)ceil_div(w, AF_TX - 2 * r), (unsigned)ceil_div(h, AT_H), (unsigned)planes);
   const int ih = (int)h, iw = (int)w;
   if (dilate) {
@@ -681,6 +921,16 @@ pg_status launch_flat2d_backward_arg(const unsigned char *code, const float *gy,
   if (planes * h * w == 0) return PG_OK;
   if (h > (1 << 30) || w > (1 << 30) || ceil_div(h, AT_H) > 65535 || planes > 65535)
     return fail(PG_ERR_INVALID_ARGUMENT, "plane too large");
+  // The 7x7 backward is so much arithmetic that the strips only win where their segments are nearly full: 256
+  // columns 690 us against 764, 320 176 / 224, but 240 102 / 98 and 160 slower still.
+  StripGeom g;
+  if (strip_geom(gy, gx, code, planes, h, w, g) && (r < 3 || (int64_t)g.segs * AS_COLS * 20 <= w * 21)) {
+    const unsigned ctas = (unsigned)ceil_div(g.units * AS_LANES, AS_THREADS);
+    if (r == 1) k_flat_bwd_arg_strip<1><<<ctas, AS_THREADS, 0, s>>>(code, gy, gx, g);
+    else if (r == 2) k_flat_bwd_arg_strip<2><<<ctas, AS_THREADS, 0, s>>>(code, gy, gx, g);
+    else k_flat_bwd_arg_strip<3><<<ctas, AS_THREADS, 0, s>>>(code, gy, gx, g);
+    return cuda_status(cudaGetLastError(), "flat morphology backward (saved arg) launch");
+  }
   const dim3 grid((unsigned)ceil_div(w, 4 * AQ_QUADS), (unsigned)ceil_div(h, AT_H), (unsigned)planes);
   // 16-byte staging: rows of whole vectors (4 floats, 4 codes) and aligned bases
   const int vec = (w % 4 == 0 && reinterpret_cast<uintptr_t>(gy) % 16 == 0 && reinterpret_cast<uintptr_t>(code) % 4 == 0)
