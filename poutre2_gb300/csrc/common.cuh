@@ -366,6 +366,10 @@ pg_status launch_reconstruction(const pg_image *markers, const pg_image *masks, 
 pg_status launch_reconstruction3d(const pg_image *marker, const pg_image &mask, const pg_image &out,
                                   const ReconRequest &rq, cudaStream_t s);
 
+// The same for volumes of 1- or 2-byte pixels whose bricks all fit on the GPU at once (recon3d_resident.cuh).
+bool try_resident3d(const pg_image *marker, const pg_image &mask, const pg_image &out, const ReconRequest &rq, cudaStream_t s,
+                    pg_status *st);
+
 pg_status create_batch_plan(const pg_image *ins, const pg_image *outs, int n, const pg_scalar &h, bool conn8, bool autotune,
                             cudaStream_t s, pg_batch_plan **out_plan);
 pg_status run_batch_plan(pg_batch_plan *p, cudaStream_t s);

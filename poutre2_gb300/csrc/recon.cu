@@ -1439,6 +1439,53 @@ __device__ __forceinline__ unsigned exch_acquire(unsigned *p, unsigned v) {
   return old;
 }
 
+// End of a resident visit, by the whole warp: marks neighbour nb of every lane with `wake` (the changed borders are
+// stored), lets tile t fall idle if it has converged and nothing beside it changed, and waits until there is
+// work.  Returns 0: visit again (the state is RS_RUNNING), 1: all tiles are idle, 2: an error was recorded.
+__device__ __forceinline__ int resident_rest(ResCtl *res, RCtl *ctl, unsigned *state, int t, int nb, bool wake,
+                                             bool converged, unsigned long long wait_ns) {
+  const int lane = threadIdx.x & 31;
+  const int n_wake = __popc(__ballot_sync(0xffffffffu, wake));
+  int off = 0;  // tiles to take off `pending` again
+  if (n_wake) {
+    if (lane == 0) atomicAdd(&res->pending, n_wake);
+    __threadfence();  // the borders and the count before the marks
+    __syncwarp();
+    const bool awake = wake && atomicExch(state + nb, RS_DIRTY) != RS_IDLE;
+    off = __popc(__ballot_sync(0xffffffffu, awake));
+  }
+  // ---- back to idle, or on with another visit
+  unsigned again = 1;
+  if (lane == 0) {
+    if (converged && atomicCAS(state + t, RS_RUNNING, RS_IDLE) == RS_RUNNING) {
+      again = 0;
+      ++off;
+    }
+    if (off && atomicSub(&res->pending, off) == off) *((volatile int *)&res->done) = 1;
+  }
+  again = __shfl_sync(0xffffffffu, again, 0);
+  int stop = 0;
+  if (lane == 0) {
+    if (!again) {
+      const unsigned long long t0 = global_ns();
+      for (unsigned polls = 0;; ++polls) {
+        if (*((volatile unsigned *)(state + t)) == RS_DIRTY) break;
+        if (polls % 8 == 7) {
+          if (*((volatile int *)&res->done)) { stop = 1; break; }
+          if (*((volatile int *)&ctl->status)) { stop = 2; break; }
+          if (wait_expired(ctl, t0, wait_ns)) { stop = 2; break; }
+        }
+        __nanosleep(polls < 16 ? 20 : 100);
+      }
+    } else if (*((volatile int *)&ctl->status)) {
+      stop = 2;
+    }
+    if (!stop) exch_acquire(state + t, RS_RUNNING);  // before the halo is read: what changes later marks again
+  }
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, stop, 0);
+}
+
 template <typename T, bool SUP, bool CONN8>
 __global__ void __launch_bounds__(kResidentWarps * 32, 1) k_reconstruct_resident(const __grid_constant__ RParams<T> P,
                                                                                 const ResTiles<T> rt) {
@@ -1542,6 +1589,7 @@ __global__ void __launch_bounds__(kResidentWarps * 32, 1) k_reconstruct_resident
   }
   const bool up = ty > 0, down = ty + 1 < im.tiles_y, west = tx > 0, east = tx + 1 < im.tiles_x;
   int visits = 0;
+  bool settled = false;  // at the local fixpoint of the last halo
   for (;;) {
     // ---- visit: the halo from the neighbours' borders
     if (++visits > P.max_rounds) {
@@ -1563,10 +1611,15 @@ __global__ void __launch_bounds__(kResidentWarps * 32, 1) k_reconstruct_resident
       }
     }
     if (CONN8) fold_halo<T, SUP>(h_top, h_bot, h_l, h_r, c_top, c_bot);
-    const uint32_t init_tb = V[0];
+    const uint32_t init_tb = V[0], tb = pk2(h_top, h_bot), lr = pk2(h_l, h_r);
     uint32_t end_lr = pub_lr;
     bool changed = false;
-    const bool converged = packed_sweeps<T, SUP, CONN8>(V, s, pk2(h_top, h_bot), pk2(h_l, h_r), P.max_sweeps, end_lr, changed);
+    // A tile at its local fixpoint moves only if its new halo moves a border pixel: most wakes end here.
+    auto pull = [&](uint32_t v, uint32_t nbv, uint32_t m) {
+      return SUP ? u16x2_min(u16x2_max(v, nbv), m) : u16x2_max(u16x2_min(v, nbv), m);
+    };
+    if (!settled || __any_sync(0xffffffffu, pull(V[0], tb, s.ma[lane]) != V[0] || pull(pub_lr, lr, s.mb[lane]) != pub_lr))
+      settled = packed_sweeps<T, SUP, CONN8>(V, s, tb, lr, P.max_sweeps, end_lr, changed);
 
     // ---- the borders that changed, and the neighbours beside them
     const uint32_t d_tb = V[0] ^ init_tb, d_lr = end_lr ^ pub_lr;
@@ -1583,44 +1636,7 @@ __global__ void __launch_bounds__(kResidentWarps * 32, 1) k_reconstruct_resident
                           : lane == 4 ? (bN & 1u) : lane == 5 ? (bN >> 31) : lane == 6 ? (bS & 1u) : (bS >> 31);
       wake = of != 0u;
     }
-    const int n_wake = __popc(__ballot_sync(0xffffffffu, wake));
-    int off = 0;  // tiles to take off `pending` again
-    if (n_wake) {
-      if (lane == 0) atomicAdd(&rt.ctl->pending, n_wake);
-      __threadfence();  // the borders and the count before the marks
-      __syncwarp();
-      const bool awake = wake && atomicExch(rt.state + nb, RS_DIRTY) != RS_IDLE;
-      off = __popc(__ballot_sync(0xffffffffu, awake));
-    }
-    // ---- back to idle, or on with another visit
-    unsigned again = 1;
-    if (lane == 0) {
-      if (converged && atomicCAS(rt.state + t, RS_RUNNING, RS_IDLE) == RS_RUNNING) {
-        again = 0;
-        ++off;
-      }
-      if (off && atomicSub(&rt.ctl->pending, off) == off) *((volatile int *)&rt.ctl->done) = 1;
-    }
-    again = __shfl_sync(0xffffffffu, again, 0);
-    int stop = 0;
-    if (lane == 0) {
-      if (!again) {
-        const unsigned long long t0 = global_ns();
-        for (unsigned polls = 0;; ++polls) {
-          if (*((volatile unsigned *)(rt.state + t)) == RS_DIRTY) break;
-          if (polls % 8 == 7) {
-            if (*((volatile int *)&rt.ctl->done)) { stop = 1; break; }
-            if (*((volatile int *)&ctl->status)) { stop = 2; break; }
-            if (wait_expired(ctl, t0, P.wait_ns)) { stop = 2; break; }
-          }
-          __nanosleep(polls < 16 ? 20 : 100);
-        }
-      } else if (*((volatile int *)&ctl->status)) {
-        stop = 2;
-      }
-      if (!stop) exch_acquire(rt.state + t, RS_RUNNING);  // before the halo is read: what changes later marks again
-    }
-    stop = __shfl_sync(0xffffffffu, stop, 0);
+    const int stop = resident_rest(rt.ctl, ctl, rt.state, t, nb, wake, settled, P.wait_ns);
     if (stop == 2) return;
     if (stop == 1) break;
   }
@@ -2200,6 +2216,8 @@ static pg_status reconstruction_noalloc(bool dilate, bool conn8, const pg_image 
 }
 
 }  // namespace pg
+
+#include "recon3d_resident.cuh"
 
 extern "C" {
 

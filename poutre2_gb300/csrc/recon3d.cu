@@ -11,23 +11,27 @@
 //               leveling, the effective mask max(marker, ref) / min(marker, ref);
 //   brick    -- a CTA loads a brick of 32 x 8 x 8 voxels of the current value (plus a one-voxel halo)
 //               and of the mask into shared memory and repeats the geodesic step on the brick, the
-//               halo held fixed, until the brick stops changing (or an iteration cap); it writes the
-//               brick to the other buffer and sets a change flag when any voxel differs from its
-//               input.  Every update is a geodesic step from a lower bound of the fixpoint (monotone
-//               and below it), so the order is immaterial; a launch that changes nothing is the
-//               fixpoint.  One launch carries values across a whole brick, where a plain step moves
-//               them one voxel;
+//               halo held fixed, until the brick stops changing (or an iteration cap), and writes it
+//               back.  Every update is a geodesic step from a lower bound of the fixpoint (monotone
+//               and below it), so the order is immaterial, and so is whether a halo voxel that another
+//               brick is writing is read old or new: a brick marks the bricks beside its changed faces
+//               (itself at the cap) for the next launch, and a launch leaves unmarked bricks alone;
 //   epilogue -- the reconstruction itself, its clip to the leveling reference, or the binary
 //               h-maxima output ref > rec.
 // The host runs the launches in batches of kStepBatch between two reads of the flag; a launch that
-// changes nothing is a fixpoint, and after at most (voxels + 1) launches one always is (each launch
-// does at least one geodesic step everywhere).
+// marks nothing has found the fixpoint, and after at most (voxels + 1) launches one always does (each
+// does at least one geodesic step wherever one is due).
+// 80 x 160 x 208 f32, a marker at half the mask: with every brick loaded and written by every launch, into a
+// second buffer, 1597 us; 1405 now.  Volumes of 1- or 2-byte voxels that fit on the GPU take
+// recon3d_resident.cuh instead.
+#include <utility>
+
 #include "common.cuh"
 
 namespace pg {
 namespace {
 
-constexpr int kStepBatch = 2;
+constexpr int kStepBatch = 4;
 constexpr int kBX = 32, kBY = 8, kBZ = 8;  // brick
 constexpr int kBrickIters = 2 * (kBX + kBY + kBZ);  // local iteration cap per launch
 
@@ -53,10 +57,19 @@ __global__ void k_r3_prep(const T *__restrict__ ref, const T *__restrict__ marke
   }
 }
 
+// loads past L1: other CTAs of the launch may be writing these voxels
+template <typename T> __device__ __forceinline__ T ld_l2(const T *p) {
+  if constexpr (std::is_same_v<T, int64_t>) return (T)__ldcg(reinterpret_cast<const long long *>(p));
+  else return __ldcg(p);
+}
+
 template <typename T, bool SUP>
-__global__ void __launch_bounds__(kBX * kBY) k_r3_brick(const T *__restrict__ cur, const T *__restrict__ mask,
-                                                        T *__restrict__ next, int D, int H, int W,
+__global__ void __launch_bounds__(kBX * kBY) k_r3_brick(T *cur, const T *__restrict__ mask, int D, int H, int W,
+                                                        unsigned char *marked, unsigned char *mark_next,
                                                         int *__restrict__ changed) {
+  const int bid = (int)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
+  if (!marked[bid]) return;  // uniform: only this CTA changes its own mark in this launch, below a barrier
+  __shared__ unsigned s_faces;
   constexpr int HX = kBX + 2, HY = kBY + 2, HZ = kBZ + 2;
   __shared__ T sr[HZ][HY][HX];      // current value with a one-voxel halo
   __shared__ T sk[kBZ][kBY][kBX];   // mask of the brick
@@ -64,10 +77,11 @@ __global__ void __launch_bounds__(kBX * kBY) k_r3_brick(const T *__restrict__ cu
   const int x0 = blockIdx.x * kBX, y0 = blockIdx.y * kBY, z0 = blockIdx.z * kBZ;
   const int64_t plane = (int64_t)H * W;
   const T NEU = Op<T, SUP>::neutral();  // never wins the extremum: voxels outside the volume
+  if (tid == 0) s_faces = 0u;
   for (int i = tid; i < HX * HY * HZ; i += kBX * kBY) {
     const int hx = i % HX, hy = (i / HX) % HY, hz = i / (HX * HY);
     const int x = x0 - 1 + hx, y = y0 - 1 + hy, z = z0 - 1 + hz;
-    sr[hz][hy][hx] = (x >= 0 && x < W && y >= 0 && y < H && z >= 0 && z < D) ? cur[z * plane + (int64_t)y * W + x] : NEU;
+    sr[hz][hy][hx] = (x >= 0 && x < W && y >= 0 && y < H && z >= 0 && z < D) ? ld_l2(cur + z * plane + (int64_t)y * W + x) : NEU;
   }
   const int x = x0 + tx, y = y0 + ty;
   const bool xy_in = x < W && y < H;
@@ -77,11 +91,13 @@ __global__ void __launch_bounds__(kBX * kBY) k_r3_brick(const T *__restrict__ cu
     sk[k][ty][tx] = (xy_in && z < D) ? mask[z * plane + (int64_t)y * W + x] : NEU;
   }
   __syncthreads();
+  if (tid == 0) marked[bid] = 0;  // every thread has read it; the next launch but one fills it again
   T start[kBZ];
 #pragma unroll
   for (int k = 0; k < kBZ; ++k) start[k] = sr[k + 1][ty + 1][tx + 1];
   // this thread's z column, updated in place (values only move towards the fixpoint, so reading a
   // neighbour's old or new value are both valid steps)
+  bool settled = false;
   for (int it = 0; it < kBrickIters; ++it) {
     bool ch = false;
     if (xy_in) {
@@ -103,20 +119,36 @@ __global__ void __launch_bounds__(kBX * kBY) k_r3_brick(const T *__restrict__ cu
         }
       }
     }
-    if (!__syncthreads_or(ch)) break;
+    if (!__syncthreads_or(ch)) {
+      settled = true;
+      break;
+    }
   }
-  bool diff = false;
+  // write back what moved; bit d: the face in direction -x +x -y +y -z +z, bit 6: the brick goes on
+  unsigned faces = settled ? 0u : 64u;
   if (xy_in) {
 #pragma unroll
     for (int k = 0; k < kBZ; ++k) {
       const int z = z0 + k;
       if (z >= D) break;
       const T v = sr[k + 1][ty + 1][tx + 1];
-      next[z * plane + (int64_t)y * W + x] = v;
-      diff |= !(v == start[k]);
+      if (v == start[k]) continue;
+      cur[z * plane + (int64_t)y * W + x] = v;
+      faces |= (tx == 0 ? 1u : 0u) | (tx == kBX - 1 ? 2u : 0u) | (ty == 0 ? 4u : 0u) | (ty == kBY - 1 ? 8u : 0u) |
+               (k == 0 ? 16u : 0u) | (k == kBZ - 1 ? 32u : 0u);
     }
   }
-  if (__any_sync(0xffffffffu, diff) && (threadIdx.x & 31) == 0) atomicOr(changed, 1);
+  faces = __reduce_or_sync(0xffffffffu, faces);
+  if ((tid & 31) == 0 && faces) atomicOr(&s_faces, faces);
+  __syncthreads();
+  if (tid < 7 && ((s_faces >> tid) & 1u)) {
+    const int dx = tid == 0 ? -1 : tid == 1 ? 1 : 0, dy = tid == 2 ? -1 : tid == 3 ? 1 : 0, dz = tid == 4 ? -1 : tid == 5 ? 1 : 0;
+    const int bx = (int)blockIdx.x + dx, by = (int)blockIdx.y + dy, bz = (int)blockIdx.z + dz;
+    if (bx >= 0 && by >= 0 && bz >= 0 && bx < (int)gridDim.x && by < (int)gridDim.y && bz < (int)gridDim.z) {
+      mark_next[(bz * (int)gridDim.y + by) * (int)gridDim.x + bx] = 1;
+      *(volatile int *)changed = 1;
+    }
+  }
 }
 
 template <typename T, bool SUP>
@@ -147,28 +179,33 @@ pg_status recon3d_t(const pg_image *marker, const pg_image &mask, const pg_image
   if (rq.init != INIT_SAT_CONST && !marker) return fail(PG_ERR_INVALID_ARGUMENT, "3D reconstruction: null marker");
   const size_t bytes = (size_t)n * sizeof(T);
   const bool own_mask = rq.init != INIT_SAT_CONST && rq.mask_mode != MASK_PLAIN;
-  Scratch bufs, emask, flag;
-  PG_TRY(bufs.alloc(2 * bytes, s));
+  const dim3 block(kBX, kBY), grid((unsigned)ceil_div(d.nx, kBX), (unsigned)ceil_div(d.ny, kBY), (unsigned)ceil_div(d.nz, kBZ));
+  const int64_t bricks = (int64_t)grid.x * grid.y * grid.z;
+  if (bricks > INT32_MAX) return fail(PG_ERR_INVALID_ARGUMENT, "3D reconstruction: volume too large");
+  Scratch buf, emask, marks, flag;
+  PG_TRY(buf.alloc(bytes, s));
   if (own_mask) PG_TRY(emask.alloc(bytes, s));
+  PG_TRY(marks.alloc(2 * (size_t)bricks, s));
   PG_TRY(flag.alloc(sizeof(int), s));
-  T *a = static_cast<T *>(bufs.ptr), *b = a + n;
+  T *a = static_cast<T *>(buf.ptr);
+  unsigned char *marked = marks.as<unsigned char>(), *mark_next = marked + bricks;
   const T *ref = static_cast<const T *>(mask.data);
   const T *eff = own_mask ? static_cast<const T *>(emask.ptr) : ref;
   int *d_flag = static_cast<int *>(flag.ptr);
+  PG_CUDA_TRY(cudaMemsetAsync(marked, 1, (size_t)bricks, s), "3D reconstruction marks");  // every brick at first
+  PG_CUDA_TRY(cudaMemsetAsync(mark_next, 0, (size_t)bricks, s), "3D reconstruction marks");
   k_r3_prep<T, SUP><<<flat_grid(n), 256, 0, s>>>(ref, marker ? static_cast<const T *>(marker->data) : nullptr,
                                                  own_mask ? static_cast<T *>(emask.ptr) : nullptr, a, n, rq.init,
                                                  rq.mask_mode, scalar_as<T>(rq.h));
   PG_CUDA_TRY(cudaGetLastError(), "3D reconstruction prep launch");
-  const dim3 block(kBX, kBY), grid((unsigned)ceil_div(d.nx, kBX), (unsigned)ceil_div(d.ny, kBY), (unsigned)ceil_div(d.nz, kBZ));
   const int64_t max_steps = n + kStepBatch + 1;
   int64_t steps = 0;
   for (;;) {
-    PG_CUDA_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), s), "3D reconstruction flag reset");
     for (int k = 0; k < kStepBatch; ++k) {
-      k_r3_brick<T, SUP><<<grid, block, 0, s>>>(a, eff, b, (int)d.nz, (int)d.ny, (int)d.nx, d_flag);
-      T *t = a;
-      a = b;
-      b = t;
+      // the batch's last launch alone decides: what it marks is due in the next
+      if (k == kStepBatch - 1) PG_CUDA_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), s), "3D reconstruction flag reset");
+      k_r3_brick<T, SUP><<<grid, block, 0, s>>>(a, eff, (int)d.nz, (int)d.ny, (int)d.nx, marked, mark_next, d_flag);
+      std::swap(marked, mark_next);
     }
     PG_CUDA_TRY(cudaGetLastError(), "3D reconstruction brick launch");
     steps += kStepBatch;
@@ -187,6 +224,8 @@ pg_status recon3d_t(const pg_image *marker, const pg_image &mask, const pg_image
 pg_status launch_reconstruction3d(const pg_image *marker, const pg_image &mask, const pg_image &out,
                                   const ReconRequest &rq, cudaStream_t s) {
   if (mask.rank != 3) return fail(PG_ERR_INVALID_ARGUMENT, "3D reconstruction of a non-3D image");
+  pg_status st = PG_OK;
+  if (try_resident3d(marker, mask, out, rq, s, &st)) return st;
   PG_DISPATCH_PTYPE(mask.ptype, T, {
     return rq.dilate ? recon3d_t<T, true>(marker, mask, out, rq, s) : recon3d_t<T, false>(marker, mask, out, rq, s);
   });
