@@ -189,14 +189,13 @@ __device__ __forceinline__ void column_windows(uint32_t *col, int ga, int half) 
   }
 }
 
-// This lane's four words from the aligned address of row byte `a` on, for a row of words that may reach
-// beyond the image's bytes [base, end): the bytes of a word across an end come one by one.
-__device__ __noinline__ uint4 edge_words(uintptr_t a, uintptr_t base, uintptr_t end) {
-  const uintptr_t p = (a & ~(uintptr_t)3) + 16u * (threadIdx.x & 31);
+// Four words from aligned address p on, `step` bytes apart, of a row that may reach beyond the image's bytes
+// [base, end): the bytes of a word across an end come one by one.
+__device__ __noinline__ uint4 edge_words(uintptr_t p, int step, uintptr_t base, uintptr_t end) {
   uint32_t w[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const uintptr_t pw = p + 4u * j;
+    const uintptr_t pw = p + (uintptr_t)(step * j);
     w[j] = 0u;
     if (pw >= base && pw + 4 <= end) {
       w[j] = __ldg(reinterpret_cast<const uint32_t *>(pw));
@@ -247,10 +246,14 @@ template <typename T> struct TileStore {
 // Rows [0, rows) of a tile: row r starts at pixel x_top + lean * r of image row y_top + r; its words go to
 // s_w[r][..] as forward windows of wlen pixels, those outside the image neutral.  Two rows at a time per warp,
 // so that the loads of both are in flight.
-template <typename T, bool SUP>
-__device__ __forceinline__ void window_rows(const T *in, int64_t H, int64_t W, int64_t y_top, int64_t x_top, int lean,
-                                            int rows, int wlen, uint32_t *s_w) {
+// Lane l holds words 4l .. 4l + 3 of a row, where the windows' shifts are cheap; PLAIN (wlen == 1, nothing to
+// shift) words l, l + 32, l + 64 and l + 96, whose loads and stores are one 128-byte line each at any alignment
+// (3000 x 3500 f32, 45 degrees, 41 pixels: 37 -> 34 us a pass).
+template <typename T, bool SUP, bool PLAIN>
+__device__ __forceinline__ void window_rows_as(const T *in, int64_t H, int64_t W, int64_t y_top, int64_t x_top, int lean,
+                                               int rows, int wlen, uint32_t *s_w) {
   constexpr int S = (int)sizeof(T), E = 4 / S;
+  constexpr int LW = PLAIN ? 1 : 4, JW = PLAIN ? 32 : 1;  // word of (lane l, j): LW * l + JW * j
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t NEU = splat<T>(Op<T, SUP>::neutral());
   const intptr_t pitch = (intptr_t)(W + lean) * S;  // bytes from a tile row to the next
@@ -272,16 +275,16 @@ __device__ __forceinline__ void window_rows(const T *in, int64_t H, int64_t W, i
       const uintptr_t aq = a + q * kWWarps * pitch, seg = aq & ~(uintptr_t)3;
       if (r < r_lo || r >= r_hi) continue;
       if (safe || (seg >= base && seg + kWRow * 4 <= end)) {
-        const uintptr_t p = seg + 16u * lane;  // this lane's words
-        if ((aq & 12u) == 0) {
+        const uintptr_t p = seg + 4u * LW * lane;  // this lane's words
+        if (!PLAIN && (aq & 12u) == 0) {
           const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
           w[q][0] = v.x; w[q][1] = v.y; w[q][2] = v.z; w[q][3] = v.w;
         } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) w[q][j] = __ldg(reinterpret_cast<const uint32_t *>(p) + j);
+          for (int j = 0; j < 4; ++j) w[q][j] = __ldg(reinterpret_cast<const uint32_t *>(p) + JW * j);
         }
       } else {
-        const uint4 v = edge_words(aq, base, end);
+        const uint4 v = edge_words(seg + 4u * LW * lane, 4 * JW, base, end);
         w[q][0] = v.x; w[q][1] = v.y; w[q][2] = v.z; w[q][3] = v.w;
       }
     }
@@ -289,37 +292,67 @@ __device__ __forceinline__ void window_rows(const T *in, int64_t H, int64_t W, i
     for (int q = 0; q < 2; ++q) {
       const int r = r0 + q * kWWarps;
       if (r >= rows) break;
+      uint32_t *row = s_w + r * kWRow + LW * lane;
+      auto store = [&](const uint4 &o) {
+        if constexpr (PLAIN) {
+          row[0] = o.x;
+          row[JW] = o.y;
+          row[2 * JW] = o.z;
+          row[3 * JW] = o.w;
+        } else {
+          *reinterpret_cast<uint4 *>(row) = o;
+        }
+      };
       if (r < r_lo || r >= r_hi) {
-        *reinterpret_cast<uint4 *>(s_w + r * kWRow + lane * 4) = make_uint4(NEU, NEU, NEU, NEU);
+        store(make_uint4(NEU, NEU, NEU, NEU));
         continue;
       }
       const unsigned sh = (unsigned)((a + q * kWWarps * pitch) & 3u) * 8u;
       if (S < 4 && sh) {
-        // the last word of lane 31 lacks its upper pixels: no output of the tile needs them (vw)
-        const uint32_t n = from_lane(w[q][0], 1);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) w[q][j] = __funnelshift_r(w[q][j], j < 3 ? w[q][j + 1] : n, sh);
-      }
-      if (clipped) {
-        // the lane's pixels [lo, hi) lie in the image
-        const int64_t x = x_top + (int64_t)lean * r + lane * 4 * E;
-        const int lo = (int)min(max(-x, (int64_t)0), (int64_t)4 * E), hi = (int)min(max(W - x, (int64_t)0), (int64_t)4 * E);
+        // the row's last word lacks its upper pixels: no output of the tile needs them (vw)
+        uint32_t n[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int l = min(max(lo - j * E, 0), E), k = min(max(hi - j * E, 0), E);  // of word j
+          if constexpr (PLAIN) {
+            n[j] = from_lane(w[q][j], 1);
+            if (j < 3) {
+              const uint32_t first = __shfl_sync(0xffffffffu, w[q][j + 1], 0);
+              if (lane == 31) n[j] = first;
+            }
+          } else {
+            n[j] = j < 3 ? w[q][j + 1] : from_lane(w[q][0], 1);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[q][j] = __funnelshift_r(w[q][j], n[j], sh);
+      }
+      if (clipped) {
+        // pixels [lo, hi) of the row lie in the image
+        const int64_t x = x_top + (int64_t)lean * r;
+        const int lo = (int)min(max(-x, (int64_t)0), (int64_t)kWRow * E), hi = (int)min(max(W - x, (int64_t)0), (int64_t)kWRow * E);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int px = (LW * lane + JW * j) * E;
+          const int l = min(max(lo - px, 0), E), k = min(max(hi - px, 0), E);  // of this word
           const uint32_t in_m = (uint32_t)(((1ull << (8 * S * k)) - 1ull) & ~((1ull << (8 * S * l)) - 1ull));
           w[q][j] = (w[q][j] & in_m) | (NEU & ~in_m);
         }
       }
       uint4 o = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
-      if (wlen > 1) {
+      if constexpr (!PLAIN) {
         RowRegs<T> m = RowRegs<T>::of(w[q]), res = m;
         row_steps<T, SUP, 1>(m, res, wlen);
         o = res.words();
       }
-      *reinterpret_cast<uint4 *>(s_w + r * kWRow + lane * 4) = o;
+      store(o);
     }
   }
+}
+template <typename T, bool SUP>
+__device__ __forceinline__ void window_rows(const T *in, int64_t H, int64_t W, int64_t y_top, int64_t x_top, int lean,
+                                            int rows, int wlen, uint32_t *s_w) {
+  if (wlen == 1) window_rows_as<T, SUP, true>(in, H, W, y_top, x_top, lean, rows, wlen, s_w);
+  else window_rows_as<T, SUP, false>(in, H, W, y_top, x_top, lean, rows, wlen, s_w);
 }
 
 template <typename T, bool SUP>
