@@ -70,43 +70,31 @@ template <bool SUP> struct Lanes<uint16_t, SUP> {
   __device__ __forceinline__ Lanes op(Lanes b) const { return {m16<SUP>(w, b.w)}; }
   __device__ __forceinline__ uint32_t word() const { return w; }
 };
+// u8: each pixel is the high byte of its lane and the low byte holds whatever lay beside it -- the min or
+// max of two 16-bit values has the min or max of their high bytes on top whatever is below, so a word IS
+// its odd pixels, one shift gives its even ones and one funnel shift a neighbour's (no byte is masked)
 template <bool SUP> struct Lanes<uint8_t, SUP> {
   uint32_t e, o;
-  static __device__ __forceinline__ Lanes at(const uint32_t *p) {
-    const uint32_t w = p[0];
-    return {__byte_perm(w, 0, 0x4240), __byte_perm(w, 0, 0x4341)};
-  }
+  static __device__ __forceinline__ Lanes of(uint32_t w) { return {w << 8, w}; }
+  static __device__ __forceinline__ Lanes at(const uint32_t *p) { return of(p[0]); }
   // even pixel 2j: window (odd 2j - 1, 2j, odd 2j + 1); odd pixel 2j + 1: (even 2j, 2j + 1, even 2j + 2)
-  static __device__ __forceinline__ Lanes hor(const uint32_t *p) {
-    const uint32_t w = p[0];
-    const uint32_t E = __byte_perm(w, 0, 0x4240), O = __byte_perm(w, 0, 0x4341);
-    const uint32_t Op = __byte_perm(p[-1], 0, 0x4341), En = __byte_perm(p[1], 0, 0x4240);
-    const uint32_t M = m16<SUP>(E, O);
-    return {m16<SUP>(M, __funnelshift_l(Op, O, 16)), m16<SUP>(M, __funnelshift_r(E, En, 16))};
+  static __device__ __forceinline__ Lanes hor(uint32_t l, uint32_t w, uint32_t r) {
+    const uint32_t M = m16<SUP>(w << 8, w);
+    return {m16<SUP>(M, __funnelshift_l(l, w, 16)), m16<SUP>(M, __funnelshift_r(w, r, 8))};
   }
+  static __device__ __forceinline__ Lanes hor(const uint32_t *p) { return hor(p[-1], p[0], p[1]); }
   static __device__ __forceinline__ void at4(const uint32_t *p, Lanes (&v)[4]) {
     const uint4 q = *reinterpret_cast<const uint4 *>(p);
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = {__byte_perm(w[k], 0, 0x4240), __byte_perm(w[k], 0, 0x4341)};
+    v[0] = of(q.x); v[1] = of(q.y); v[2] = of(q.z); v[3] = of(q.w);
   }
-  // each word split once; the left word's odd and the right word's even pixels from the neighbours
   static __device__ __forceinline__ void hor4(const uint32_t *p, Lanes (&h)[4]) {
     const uint4 q = *reinterpret_cast<const uint4 *>(p);
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-    uint32_t E[6], O[6];  // index k + 1 = word k; O[0] of the left word, E[5] of the right one
-    O[0] = __byte_perm(p[-1], 0, 0x4341);
-    E[5] = __byte_perm(p[4], 0, 0x4240);
+    const uint32_t w[6] = {p[-1], q.x, q.y, q.z, q.w, p[4]};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) { E[k + 1] = __byte_perm(w[k], 0, 0x4240); O[k + 1] = __byte_perm(w[k], 0, 0x4341); }
-#pragma unroll
-    for (int k = 1; k <= 4; ++k) {
-      const uint32_t M = m16<SUP>(E[k], O[k]);
-      h[k - 1] = {m16<SUP>(M, __funnelshift_l(O[k - 1], O[k], 16)), m16<SUP>(M, __funnelshift_r(E[k], E[k + 1], 16))};
-    }
+    for (int k = 0; k < 4; ++k) h[k] = hor(w[k], w[k + 1], w[k + 2]);
   }
   __device__ __forceinline__ Lanes op(Lanes b) const { return {m16<SUP>(e, b.e), m16<SUP>(o, b.o)}; }
-  __device__ __forceinline__ uint32_t word() const { return __byte_perm(e, o, 0x6240); }
+  __device__ __forceinline__ uint32_t word() const { return __byte_perm(e, o, 0x7351); }
 };
 // i32 / f32: one pixel per word, min / max as everywhere else (wop: signed compare, fminf / fmaxf)
 template <typename T, bool SUP> struct Lanes {
