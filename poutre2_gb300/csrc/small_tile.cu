@@ -13,8 +13,8 @@
 // tile's rows (of every slice of the tile): the left and right neighbours of each pixel come from
 // funnel shifts with the neighbouring words, the rows above and below are the next shared-memory
 // rows, and a volume's slices slide through registers.  u16 words are min / max'ed as u16x2; u8 words
-// are split once into their even and odd pixels on 16-bit lanes (the native u16x2 min / max; the
-// packed 8-bit form is emulated), combined there and merged once; i32 / f32 words hold one pixel.
+// as their even and odd pixels on 16-bit lanes (the native u16x2 min / max; the packed 8-bit form is
+// emulated), merged once; i32 / f32 words hold one pixel.
 // Pixels outside the image arrive as TMA's zero fill, the neutral value of the unsigned dilations;
 // for the other operators, tiles at the border set them to the neutral value first.  The TMA wait is
 // bounded (tile::kWaitNs); on expiry the CTA records PG_ERR_CUDA in g_small_tile_status (read by
@@ -33,8 +33,8 @@ constexpr int kSTW = 64;         // output words per tile row
 constexpr int kSTBW = kSTW + 8;  // box words: one 16-byte chunk of halo each side
 constexpr int kST2Rows = 64;     // output rows of a 2D tile (a thread per word)
 constexpr int kST2QRows = 64;    // output rows of a 2D tile (a thread per quad of words)
-// u8 images take the quad kernel (4096^2 square 12.3 -> 10.2 us); for u16 / i32 / f32 the thread per
-// word measured 1-2 % faster on 8192^2 / 16384^2 images and the same on 4096^2
+// u8 images take the quad kernel (4096^2 square 12.3 -> 10.2 us before the lanes below); for u16 / i32 /
+// f32 the thread per word measured 1-2 % faster on 8192^2 / 16384^2 images and the same on 4096^2
 template <typename T> constexpr bool kQuad2D = sizeof(T) == 1;
 constexpr int kST2QThreads = 128;  // threads of a quad tile
 constexpr int kST3Rows = 8;        // output rows of a 3D tile
@@ -72,7 +72,10 @@ template <bool SUP> struct Lanes<uint16_t, SUP> {
 };
 // u8: each pixel is the high byte of its lane and the low byte holds whatever lay beside it -- the min or
 // max of two 16-bit values has the min or max of their high bytes on top whatever is below, so a word IS
-// its odd pixels, one shift gives its even ones and one funnel shift a neighbour's (no byte is masked)
+// its odd pixels, one shift gives its even ones and one funnel shift a neighbour's (no byte is masked).  The
+// tiles of an image in L2, and those that take 27 neighbours, are bound by these operations (8 a word and
+// row pass when both halves were masked out, now 5): the 3x3x3 cube on 512^3 58.0 -> 47.8 us (39.5 at copy
+// bandwidth), on 256^3 12.2 -> 11.4, the 3x3 square on 4096^2 9.1 -> 7.6, the 3D cross on 512^3 46.2 -> 43.7
 template <bool SUP> struct Lanes<uint8_t, SUP> {
   uint32_t e, o;
   static __device__ __forceinline__ Lanes of(uint32_t w) { return {w << 8, w}; }
