@@ -61,7 +61,7 @@ template <typename T, bool SUP> struct Acc {
 };
 
 // A lane's four words of a row in registers, as NR registers of two 16-bit lanes or one 32-bit pixel:
-// u8: r[2j] = even, r[2j + 1] = odd pixels of word j (clean 16-bit lanes); others: r[j] = word j.
+// u8: r[2j] = even, r[2j + 1] = odd pixels of word j (in the high bytes, as Acc); others: r[j] = word j.
 template <typename T> struct RowRegs {
   static constexpr int NR = sizeof(T) == 1 ? 8 : 4;
   uint32_t r[NR];
@@ -70,8 +70,8 @@ template <typename T> struct RowRegs {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if constexpr (sizeof(T) == 1) {
-        o.r[2 * j] = __byte_perm(w[j], 0u, 0x4240);
-        o.r[2 * j + 1] = __byte_perm(w[j], 0u, 0x4341);
+        o.r[2 * j] = w[j] << 8;
+        o.r[2 * j + 1] = w[j];
       } else {
         o.r[j] = w[j];
       }
@@ -80,8 +80,8 @@ template <typename T> struct RowRegs {
   }
   __device__ __forceinline__ uint4 words() const {
     if constexpr (sizeof(T) == 1)
-      return make_uint4(__byte_perm(r[0], r[1], 0x6240), __byte_perm(r[2], r[3], 0x6240),
-                        __byte_perm(r[4], r[5], 0x6240), __byte_perm(r[6], r[7], 0x6240));
+      return make_uint4(__byte_perm(r[0], r[1], 0x7351), __byte_perm(r[2], r[3], 0x7351),
+                        __byte_perm(r[4], r[5], 0x7351), __byte_perm(r[6], r[7], 0x7351));
     else
       return make_uint4(r[0], r[1], r[2], r[3]);
   }
