@@ -782,14 +782,20 @@ __device__ __forceinline__ void fold_halo(T &h_top, T &h_bot, T &h_l, T &h_r, T 
   h_top = t3; h_bot = b3; h_l = l3; h_r = r3;
 }
 
+// two border pixels after their halo: the value, pulled by the halo's within the mask
+template <bool SUP> __device__ __forceinline__ uint32_t pulled(uint32_t v, uint32_t halo, uint32_t mask) {
+  return SUP ? u16x2_min(u16x2_max(v, halo), mask) : u16x2_max(u16x2_min(v, halo), mask);
+}
+
 // One visit of a packed tile: as process_tile_reg below, but the pixels stay in their own width in shared memory
 // (6.5 KB a warp for u8, five CTAs per SM) and come in whole words at any alignment.  Rows of no whole 16-byte
 // vectors were staged pixel by pixel before: 21500 of a visit's 37700 cycles in a 512-image batch (sweeps 8100),
 // now 6600 of 22300; with the runs of for_pixel_runs and a search of the images in shared memory the batch of
-// 512 u8 images of 64-1024 pixels a side takes 2.37 ms (before: 6.25), one 2048^2 u8 image 131 us a call (177).
+// 512 u8 images of 64-1024 pixels a side takes 2.24 ms (before: 6.25), one 2048^2 u8 image 131 us a call (177).
 // A visit is bound by latency: loads 6600 cycles, sweeps 7300, the fence, atomics and slot of its end 10300.
 template <typename T, bool SUP, bool CONN8>
-__device__ __forceinline__ int process_tile_packed(const RImg &im, const RParams<T> &P, int t_local, PackedTile<T> &s) {
+__device__ __forceinline__ int process_tile_packed(const RImg &im, const RParams<T> &P, int t_local, bool settled,
+                                                   PackedTile<T> &s) {
   static_assert(sizeof(T) <= 2, "two pixels per register");
   constexpr int S = (int)sizeof(T), TP = PackedTile<T>::TP;
   using OT = Op<T, SUP>;
@@ -895,6 +901,14 @@ __device__ __forceinline__ int process_tile_packed(const RImg &im, const RParams
   __syncwarp();
   if (CONN8) fold_halo<T, SUP>(h_top, h_bot, h_l, h_r, c_top, c_bot);
   const uint32_t tb = pk2(h_top, h_bot), lr = pk2(h_l, h_r);
+  // A settled tile whose halo moves nothing is done.  512 u8 images of 64-1024 pixels 2356 -> 2238 us, leveling 4096^2
+  // u8 793 -> 766; u16 has no register left for it (leveling 3000 x 4001 911 -> 948), nor have the 4-byte tiles
+  // (binary h-maxima 2048^2 f32 198 -> 211).
+  if constexpr (sizeof(T) == 1) {
+    if (settled && !__any_sync(0xffffffffu, pulled<SUP>(V[0], tb, s.ma[lane]) != V[0] ||
+                                                pulled<SUP>(init_lr, lr, s.mb[lane]) != init_lr))
+      return 0;
+  }
 
   uint32_t end_lr = init_lr;
   bool changed = false;
@@ -1118,7 +1132,7 @@ __device__ int process_tile_reg(const RImg &im, const RParams<T> &P, int t_local
 // time, through its state:
 //   IDLE --queue--> QUEUED --pop--> RUNNING --done--> IDLE (or QUEUED again if it yielded)
 //   RUNNING --a neighbour changed its border meanwhile--> DIRTY --done--> QUEUED
-// The queue is a ring of 64-bit slots (position tag << 32 | tile + 1), a multi-producer multi-
+// The queue is a ring of 64-bit slots (position tag << 32 | kSettled | tile + 1), a multi-producer multi-
 // consumer ring with sequence numbers: a popper takes a ticket with one atomicAdd on `head`
 // and waits for its slot to carry its position; a pusher takes positions with one atomicAdd
 // on `tail` and waits until the slot's previous lap was consumed (tag = position - cap, tile
@@ -1159,17 +1173,22 @@ __device__ __forceinline__ unsigned long long slot_val(unsigned pos, unsigned ti
   return ((unsigned long long)pos << 32) | tile1;
 }
 
-// Lane 0 pops ticket `pos`: the tile to visit, or -1 when the work is done or an error was recorded.  A waiting
+// In a slot's tile field: the tile's last visit ended at its local fixpoint (it was idle when a neighbour queued
+// it, or it was dirtied during that visit), so it moves only if its new halo moves a border pixel.  u8 tiles look.
+template <typename T> constexpr unsigned kSettled = sizeof(T) == 1 ? 0x80000000u : 0u;
+
+// Lane 0 pops ticket `pos`: the slot's tile field (tile + 1 and kSettled), or 0 when the work is done or an error was
+// recorded.  A waiting
 // warp polls its own slot only (every idle warp polling the shared counters as well slowed the atomics on
 // them): the warp that ends the last visit fills the slots of the tickets still out with kExit, and a warp that
 // takes its ticket later sees `pending` at zero on its first poll.
 static constexpr unsigned kExit = 0xffffffffu;
 
 template <typename T>
-__device__ int wl_pop(const WorkList<T> &wl, RCtl *ctl, unsigned pos, long long max_tickets) {
+__device__ unsigned wl_pop(const WorkList<T> &wl, RCtl *ctl, unsigned pos, long long max_tickets) {
   if ((long long)pos >= max_tickets) {  // runaway guard: far more visits than any input needs
     set_status(ctl, PG_ERR_NOT_CONVERGED);
-    return -1;
+    return 0u;
   }
   volatile unsigned long long *slot = wl.ring + pos % wl.cap;
   const unsigned long long t0 = global_ns();
@@ -1179,19 +1198,19 @@ __device__ int wl_pop(const WorkList<T> &wl, RCtl *ctl, unsigned pos, long long 
     unsigned long long tp = ~0ull;
     if (polls % 16 == 0) tp = *((volatile unsigned long long *)&wl.q->tp);  // with the slot: one round trip
     if ((unsigned)(v >> 32) == pos && (unsigned)v != 0u) break;
-    if (tp_pending(tp) == 0) return -1;
+    if (tp_pending(tp) == 0) return 0u;
     if (polls % 16 == 15) {
-      if (*((volatile int *)&ctl->status) != 0) return -1;
-      if (wait_expired(ctl, t0, wl.wait_ns)) return -1;
+      if (*((volatile int *)&ctl->status) != 0) return 0u;
+      if (wait_expired(ctl, t0, wl.wait_ns)) return 0u;
     }
     __nanosleep(polls < 8 ? 40 : 200);
   }
-  if ((unsigned)v == kExit) return -1;
+  if ((unsigned)v == kExit) return 0u;
   *slot = slot_val(pos, 0u);  // consumed: the next lap's pusher may write
-  const unsigned tile = (unsigned)v - 1u;
+  const unsigned tile = ((unsigned)v & ~kSettled<T>) - 1u;
   *((volatile unsigned *)(wl.state + tile)) = TS_RUNNING;  // QUEUED until now: nobody else moves it
   __threadfence();  // the neighbours' pixels written before they queued this tile
-  return (int)tile;
+  return (unsigned)v;
 }
 
 // Retry limit of the state-change loops below: a retry means another warp changed the same
@@ -1269,7 +1288,8 @@ __device__ void wl_finish(const WorkList<T> &wl, RCtl *ctl, const RImg &im, int 
         if (wait_expired(ctl, t0, wl.wait_ns)) break;
       }
     }
-    *slot = slot_val(pos, (unsigned)cand + 1u);
+    // a neighbour pushed here was idle: its last visit had settled; this tile settled unless it yielded
+    *slot = slot_val(pos, ((unsigned)cand + 1u) | (self && yielded ? 0u : kSettled<T>));
   }
   if (left == 0) {  // the last visit: release the warps that wait (tickets from the tail on)
     unsigned head = 0;
@@ -1373,15 +1393,17 @@ __global__ void __launch_bounds__(kRegWarps * 32, sizeof(T) <= 2 ? 5 : 4) k_reco
   // positions
   const long long max_tickets = std::min<long long>((long long)P.ntiles * P.max_rounds, (1ll << 31) - 2ll * P.ntiles);
   for (unsigned ticket = (unsigned)(tid >> 5);;) {
-    int t = -1;
-    if (lane == 0) t = wl_pop(wl, ctl, ticket, max_tickets);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (t < 0) break;
+    unsigned popped = 0u;
+    if (lane == 0) popped = wl_pop(wl, ctl, ticket, max_tickets);
+    popped = __shfl_sync(0xffffffffu, popped, 0);
+    if (popped == 0u) break;
+    const int t = (int)((popped & ~kSettled<T>) - 1u);
+    const bool settled = (popped & kSettled<T>) != 0u;
     int tl = 0;
     const RImg &im = image_of(P, t, tl, begin);
     int f;
     if constexpr (sizeof(T) <= 2) {
-      f = process_tile_packed<T, SUP, CONN8>(im, P, tl, *reinterpret_cast<PackedTile<T> *>(s_raw[warp]));
+      f = process_tile_packed<T, SUP, CONN8>(im, P, tl, settled, *reinterpret_cast<PackedTile<T> *>(s_raw[warp]));
     } else {
       T *s_m = reinterpret_cast<T *>(s_raw[warp]);
       f = process_tile_reg<T, SUP, CONN8>(im, P, tl, s_m, s_m + 32 * kRP);
@@ -1615,10 +1637,8 @@ __global__ void __launch_bounds__(kResidentWarps * 32, 1) k_reconstruct_resident
     uint32_t end_lr = pub_lr;
     bool changed = false;
     // A tile at its local fixpoint moves only if its new halo moves a border pixel: most wakes end here.
-    auto pull = [&](uint32_t v, uint32_t nbv, uint32_t m) {
-      return SUP ? u16x2_min(u16x2_max(v, nbv), m) : u16x2_max(u16x2_min(v, nbv), m);
-    };
-    if (!settled || __any_sync(0xffffffffu, pull(V[0], tb, s.ma[lane]) != V[0] || pull(pub_lr, lr, s.mb[lane]) != pub_lr))
+    if (!settled || __any_sync(0xffffffffu, pulled<SUP>(V[0], tb, s.ma[lane]) != V[0] ||
+                                                pulled<SUP>(pub_lr, lr, s.mb[lane]) != pub_lr))
       settled = packed_sweeps<T, SUP, CONN8>(V, s, tb, lr, P.max_sweeps, end_lr, changed);
 
     // ---- the borders that changed, and the neighbours beside them
