@@ -23,7 +23,7 @@
 // 0.80 ms on a thresholded 2048^2 u8 image, nearly all of it in long chains of dependent loads
 // contending for the same few roots; a tile's chains are in shared memory, and one pixel in forty
 // reaches global memory.  2048^2 u8 binary: tile 25 us,
-// border 14, flatten 6, number 4, resolve 11; 83 us a call with the count's read back, against 800.
+// border 14, flatten 6, number 4, resolve 11; 77 us a call with the count's read back, against 800.
 // The floor (input read, labels written) is 5.6 us; the tile pass is bound by the dependent shared-memory
 // loads of the runs (40 % of the issue slots), border and flatten by the L2 latency of their chains.
 //

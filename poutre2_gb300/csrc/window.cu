@@ -24,7 +24,7 @@
 //
 // Bound: the ALU pipe (min / max, shifts and byte permutes all issue there at half rate; 54 % busy at 2999 x
 // 4001 u8, 21x21) and the waits of the 24 warps an image of that size gives an SM; the input is read from
-// DRAM once, the halo from L2.  2999 x 4001 u8: 21x21 120 -> 29 us, 45-degree segment of 21 90 -> 21 us (pixel-
+// DRAM once, the halo from L2.  2999 x 4001 u8: 21x21 120 -> 26 us, 45-degree segment of 21 90 -> 19 us (pixel-
 // wise van Herk in shared memory before: rows of no whole words); f32 4096^2 45 degrees of 21 104 -> 43 us.
 #include <algorithm>
 #include <atomic>
@@ -454,7 +454,7 @@ pg_status window_t(const pg_image &in, const pg_image &out, WindowGeom g, cudaSt
 // shared memory as windows of the chord's length, moved by its first column (the loads take any alignment),
 // and every thread adds the chords' rows to its R outputs, kept in registers.
 // Bound: the ALU pipe, 4-5 instructions per chord and word of outputs plus a row pass per group.  2048^2 u8,
-// radius 7: 905 us (149 bounds-checked loads per pixel, small_se.cu) -> 29 us; radius 2 f32 121 -> 25 us.
+// radius 7: 905 us (149 bounds-checked loads per pixel, small_se.cu) -> 31 us; radius 2 f32 121 -> 25 us.
 struct ChordGroup {
   int x0;                  // first column of the chords
   short dz, len;           // slice, pixels
