@@ -116,8 +116,14 @@ pg_status pg_check_device(pg_stream_t stream) {
   HostSlot slot;
   bool queued = false;
   if (capture == cudaStreamCaptureStatusNone && slot.word) {
-    k_read_status<<<1, 32, 0, s>>>(w, slot.word);
-    queued = cudaGetLastError() == cudaSuccess;  // not, for instance, on another device's stream
+    // The launch's own result: cudaGetLastError would also return an error some earlier call left behind, and the
+    // word that this kernel reads and clears would then be lost.
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(1);
+    cfg.blockDim = dim3(32);
+    cfg.stream = s;
+    queued = cudaLaunchKernelEx(&cfg, k_read_status, w, slot.word) == cudaSuccess;  // not on another device's stream
+    if (!queued) (void)cudaGetLastError();
   }
   PG_CUDA_TRY(cudaStreamSynchronize(s), "stream synchronisation");
   if (queued) {

@@ -1,0 +1,66 @@
+"""What a kernel recorded reaches the caller of pg_check_device, whatever other calls left behind."""
+import ctypes
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+NOT_CONVERGED = 9
+
+
+@pytest.fixture()
+def L():
+    from poutre2_gb300 import _lib
+    lib = _lib.load()
+    yield lib
+    assert lib.pg_debug_set_limits(0, 0) == 0
+    from poutre2_gb300.image import descriptor
+    a, b = (torch.zeros(8, 8, dtype=torch.uint8, device="cuda") for _ in range(2))
+    da, db = descriptor(a), descriptor(b)
+    for _ in range(2):  # the first kernel launch after a pending error reports it
+        status = lib.pg_erode(ctypes.byref(da), 2, 1, ctypes.byref(db), None)
+    assert status == 0
+
+
+def leave_an_error_pending(L):
+    """A call that is refused while a stream captures leaves its error with the CUDA runtime of the library: no
+    later call of it failed.  The capture ends without a graph."""
+    driver = ctypes.CDLL("libcuda.so.1")
+    stream, graph = torch.cuda.Stream(), ctypes.c_void_p()
+    torch.cuda.synchronize()
+    assert driver.cuStreamBeginCapture_v2(ctypes.c_void_p(stream.cuda_stream), 0) == 0
+    assert L.pg_last_reconstruction_rounds() == -1
+    driver.cuStreamEndCapture(ctypes.c_void_p(stream.cuda_stream), ctypes.byref(graph))
+    assert not graph.value
+
+
+def capped_reconstruction(L):
+    """Queues a reconstruction that gives up after one visit a tile."""
+    from poutre2_gb300.image import descriptor
+    f = np.zeros((256, 256), np.uint8)
+    f[::4] = 100
+    f[2::8, -1] = f[1::8, -1] = f[3::8, -1] = 100
+    f[6::8, 0] = f[5::8, 0] = f[7::8, 0] = 100
+    m = np.zeros_like(f)
+    m[0, 0] = 100
+    k, mk = torch.from_numpy(f).cuda(), torch.from_numpy(m).cuda()
+    out = torch.empty_like(k)
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    d = [descriptor(x) for x in (mk, k, out)]
+    assert L.pg_debug_set_limits(1, 0) == 0
+    assert L.pg_reconstruction(1, ctypes.byref(d[0]), ctypes.byref(d[1]), 2, ctypes.byref(d[2]), s) == 0
+    assert L.pg_debug_set_limits(0, 0) == 0
+    torch.cuda.synchronize()
+    return s
+
+
+def test_a_status_is_kept_while_an_older_error_is_pending(L):
+    capped_reconstruction(L)  # the kernels are loaded
+    L.pg_check_device(ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    leave_an_error_pending(L)
+    s = capped_reconstruction(L)
+    assert L.pg_check_device(s) == NOT_CONVERGED
+    assert L.pg_check_device(s) == 0  # reported once
