@@ -615,8 +615,10 @@ bool try_window(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx,
   WindowGeom g{};
   g.H = d.ny;
   g.W = d.nx;
-  g.hx = (int)hx;
-  g.hy = (int)hy;
+  // clipped windows reach no further than the image: on one column (row) they are the pixels themselves, with no
+  // neutral value beside them to stand in for an infinity
+  g.hx = (int)std::min(hx, d.nx - 1);
+  g.hy = (int)std::min(hy, d.ny - 1);
   g.lean = lean;
   switch (in.ptype) {
     case PG_PTYPE_U8: *st = dilate ? window_t<uint8_t, true>(in, out, g, s) : window_t<uint8_t, false>(in, out, g, s); return true;
