@@ -1443,11 +1443,17 @@ __global__ void __launch_bounds__(kRegWarps * 32, sizeof(T) <= 2 ? 5 : 4) k_reco
 enum : unsigned { RS_IDLE = 0, RS_RUNNING = 1, RS_DIRTY = 2 };
 static constexpr int kResidentWarps = 32;
 
+// `pending` (low half of `work`) shares its word with a count of the visits that woke a tile or fell idle (high
+// half), so that a waiting tile can tell a long propagation elsewhere from one that stands still.
 struct ResCtl {  // in the work area, cleared before the launch
-  int pending, pad0[31];
+  unsigned long long work;
+  int pad0[30];
   int done, pad1[31];
 };
 static_assert(sizeof(ResCtl) == 256, "ResCtl layout");
+__device__ __forceinline__ unsigned res_progress(const ResCtl *res) {
+  return (unsigned)(*((volatile const unsigned long long *)&res->work) >> 32);
+}
 
 template <typename T> struct ResTiles {
   ResCtl *ctl;
@@ -1464,13 +1470,15 @@ __device__ __forceinline__ unsigned exch_acquire(unsigned *p, unsigned v) {
 // End of a resident visit, by the whole warp: marks neighbour nb of every lane with `wake` (the changed borders are
 // stored), lets tile t fall idle if it has converged and nothing beside it changed, and waits until there is
 // work.  Returns 0: visit again (the state is RS_RUNNING), 1: all tiles are idle, 2: an error was recorded.
+// The wait gives up when its limit passes with no progress anywhere; a tile that a front reaches late may have to
+// wait longer than that (the limit alone, counted from falling idle, refused paths of more than 4 s).
 __device__ __forceinline__ int resident_rest(ResCtl *res, RCtl *ctl, unsigned *state, int t, int nb, bool wake,
                                              bool converged, unsigned long long wait_ns) {
   const int lane = threadIdx.x & 31;
   const int n_wake = __popc(__ballot_sync(0xffffffffu, wake));
   int off = 0;  // tiles to take off `pending` again
   if (n_wake) {
-    if (lane == 0) atomicAdd(&res->pending, n_wake);
+    if (lane == 0) atomicAdd(&res->work, (1ull << 32) + (unsigned)n_wake);
     __threadfence();  // the borders and the count before the marks
     __syncwarp();
     const bool awake = wake && atomicExch(state + nb, RS_DIRTY) != RS_IDLE;
@@ -1483,19 +1491,30 @@ __device__ __forceinline__ int resident_rest(ResCtl *res, RCtl *ctl, unsigned *s
       again = 0;
       ++off;
     }
-    if (off && atomicSub(&res->pending, off) == off) *((volatile int *)&res->done) = 1;
+    // less `off` in the low half carries one into the high half
+    if (off && (unsigned)atomicAdd(&res->work, (1ull << 32) - (unsigned)off) == (unsigned)off) *((volatile int *)&res->done) = 1;
   }
   again = __shfl_sync(0xffffffffu, again, 0);
   int stop = 0;
   if (lane == 0) {
     if (!again) {
-      const unsigned long long t0 = global_ns();
+      unsigned long long t0 = global_ns();
+      unsigned seen = ~0u;
       for (unsigned polls = 0;; ++polls) {
         if (*((volatile unsigned *)(state + t)) == RS_DIRTY) break;
         if (polls % 8 == 7) {
           if (*((volatile int *)&res->done)) { stop = 1; break; }
           if (*((volatile int *)&ctl->status)) { stop = 2; break; }
-          if (wait_expired(ctl, t0, wait_ns)) { stop = 2; break; }
+          if (global_ns() - t0 > wait_ns) {
+            const unsigned now = res_progress(res);  // looked at once a limit: idle polls leave the counter's line alone
+            if (now == seen) {
+              set_status(ctl, PG_ERR_NOT_CONVERGED);
+              stop = 2;
+              break;
+            }
+            seen = now;
+            t0 = global_ns();
+          }
         }
         __nanosleep(polls < 16 ? 20 : 100);
       }
@@ -1595,7 +1614,7 @@ __global__ void __launch_bounds__(kResidentWarps * 32, 1) k_reconstruct_resident
     if (lane == 0) rt.state[t] = RS_RUNNING;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    rt.ctl->pending = P.ntiles;
+    rt.ctl->work = (unsigned)P.ntiles;
     g_recon_rounds = 0;
   }
   if (!grid_barrier(ctl, P.wait_ns)) return;

@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(brick_warps<T>() * 32, 1) k_r3_resident(const 
     if (lane == 0) P.state[t] = RS_RUNNING;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    P.res->pending = P.bricks;
+    P.res->work = (unsigned)P.bricks;
     g_recon_rounds = 0;
   }
   if (!grid_barrier(ctl, P.wait_ns)) return;
