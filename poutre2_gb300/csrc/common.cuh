@@ -183,12 +183,12 @@ struct Scratch {
 
 // One 8-byte word of pinned host memory that kernels write and the host reads after synchronising their
 // stream (status.cu): a result comes back without a copy call.  The words are a fixed set of kHostSlots per
-// process, shared by all threads; `word` is null while all of them are taken (or none could be made), and the
-// caller then copies from device memory.
+// process, shared by all threads; `word` is null while all of them are taken, if none could be made, or if none
+// is wanted, and the caller then copies from device memory.
 constexpr int kHostSlots = 64;
 class HostSlot {
  public:
-  HostSlot();
+  explicit HostSlot(bool wanted);
   ~HostSlot();
   HostSlot(const HostSlot &) = delete;
   HostSlot &operator=(const HostSlot &) = delete;

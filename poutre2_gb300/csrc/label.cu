@@ -565,9 +565,10 @@ pg_status label_t(const pg_image &in, const pg_image &out, unsigned edges, int64
   int32_t *par = work.as<int32_t>();
   unsigned *roots = reinterpret_cast<unsigned *>(work.as<char>() + par_bytes);
   int32_t *cnt = reinterpret_cast<int32_t *>(work.as<char>() + par_bytes + root_bytes);
-  HostSlot slot;  // the count goes straight to the host, where one waits for it
+  // the count goes straight to the host, where one waits for it (without one the call can be captured)
+  HostSlot slot(count != nullptr);
   long long *device_total = reinterpret_cast<long long *>(cnt + kLSegments);
-  long long *total = count && slot.word ? slot.word : device_total;
+  long long *total = slot.word ? slot.word : device_total;
   int64_t *o = static_cast<int64_t *>(out.data);
   const T *src = static_cast<const T *>(in.data);
   PG_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)nseg, s), "clear label counts");

@@ -18,25 +18,29 @@ struct SlotPool {
   std::atomic<uint64_t> taken{0};
 };
 
-// Made on first use and kept for the life of the process (512 bytes); `host` stays null if that fails.
-SlotPool &slots() {
+// Made on first use and kept for the life of the process (512 bytes); null where that fails, as it does while a
+// stream capture of another thread forbids the allocation: the next caller tries again.
+SlotPool *slots() {
   static SlotPool pool;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void *h = nullptr, *d = nullptr;
-    if (cudaHostAlloc(&h, kHostSlots * sizeof(long long), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return;
-    }
-    if (cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess) {
-      (void)cudaGetLastError();
-      cudaFreeHost(h);
-      return;
-    }
-    pool.host = static_cast<long long *>(h);
-    pool.device = static_cast<long long *>(d);
-  });
-  return pool;
+  static std::mutex mu;
+  static std::atomic<bool> made{false};
+  if (made.load()) return &pool;
+  std::lock_guard<std::mutex> lk(mu);
+  if (made.load()) return &pool;
+  void *h = nullptr, *d = nullptr;
+  if (cudaHostAlloc(&h, kHostSlots * sizeof(long long), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  if (cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess) {
+    (void)cudaGetLastError();
+    cudaFreeHost(h);
+    return nullptr;
+  }
+  pool.host = static_cast<long long *>(h);
+  pool.device = static_cast<long long *>(d);
+  made.store(true);
+  return &pool;
 }
 
 constexpr int kWords = 7;
@@ -61,24 +65,24 @@ __global__ void k_read_status(StatusWords w, long long *result) {
 
 }  // namespace
 
-HostSlot::HostSlot() {
-  SlotPool &pool = slots();
-  if (!pool.host) return;
-  uint64_t t = pool.taken.load();
+HostSlot::HostSlot(bool wanted) {
+  SlotPool *pool = wanted ? slots() : nullptr;
+  if (!pool) return;
+  uint64_t t = pool->taken.load();
   while (t != ~0ull) {
     const int i = __builtin_ctzll(~t);
-    if (pool.taken.compare_exchange_weak(t, t | (1ull << i))) {
+    if (pool->taken.compare_exchange_weak(t, t | (1ull << i))) {
       index_ = i;
-      word = pool.device + i;
+      word = pool->device + i;
       break;
     }
   }
   static_assert(kHostSlots == 64, "one bit per word");
 }
 HostSlot::~HostSlot() {
-  if (index_ >= 0) slots().taken.fetch_and(~(1ull << index_));
+  if (index_ >= 0) slots()->taken.fetch_and(~(1ull << index_));
 }
-long long HostSlot::value() const { return *const_cast<volatile long long *>(slots().host + index_); }
+long long HostSlot::value() const { return *const_cast<volatile long long *>(slots()->host + index_); }
 
 }  // namespace pg
 
@@ -113,9 +117,9 @@ pg_status pg_check_device(pg_stream_t stream) {
     (void)cudaGetLastError();
     capture = cudaStreamCaptureStatusActive;
   }
-  HostSlot slot;
+  HostSlot slot(capture == cudaStreamCaptureStatusNone);  // its pool's allocation would break a capture
   bool queued = false;
-  if (capture == cudaStreamCaptureStatusNone && slot.word) {
+  if (slot.word) {
     // The launch's own result: cudaGetLastError would also return an error some earlier call left behind, and the
     // word that this kernel reads and clears would then be lost.
     cudaLaunchConfig_t cfg{};
