@@ -585,7 +585,12 @@ pg_status label_t(const pg_image &in, const pg_image &out, unsigned edges, int64
   const unsigned rg = (unsigned)ceil_div(n, 4 * kLThreads);
   if (reinterpret_cast<uintptr_t>(o) % 16 == 0) k_label_resolve<true><<<rg, kLThreads, 0, s>>>(par, n, o);
   else k_label_resolve<false><<<rg, kLThreads, 0, s>>>(par, n, o);
-  PG_TRY(cuda_status(cudaGetLastError(), "labelling kernels launch"));
+  const pg_status launched = cuda_status(cudaGetLastError(), "labelling kernels launch");
+  if (launched != PG_OK) {
+    // the kernels that were launched may still write the word: it goes back to the pool after them
+    if (total != device_total) (void)cudaStreamSynchronize(s);
+    return launched;
+  }
   if (count) {
     if (total == device_total)
       PG_CUDA_TRY(cudaMemcpyAsync(count, total, sizeof(int64_t), cudaMemcpyDeviceToHost, s), "label count copy");

@@ -64,3 +64,21 @@ def test_a_status_is_kept_while_an_older_error_is_pending(L):
     s = capped_reconstruction(L)
     assert L.pg_check_device(s) == NOT_CONVERGED
     assert L.pg_check_device(s) == 0  # reported once
+
+
+def test_a_failed_labelling_keeps_its_word_until_its_kernels_ended(L):
+    # the call reports the pending error after its kernels were queued behind a long one: when it returns, none of
+    # them can still write the count into a pinned word that another call has been given meanwhile
+    from poutre2_gb300.image import descriptor
+    x = torch.ones(64, 64, dtype=torch.uint8, device="cuda")
+    out = torch.empty(64, 64, dtype=torch.int64, device="cuda")
+    dx, do, count = descriptor(x), descriptor(out), ctypes.c_int64(-1)
+    stream = torch.cuda.Stream()
+    s = ctypes.c_void_p(stream.cuda_stream)
+    assert L.pg_label_binary(ctypes.byref(dx), 2, ctypes.byref(do), ctypes.byref(count), s) == 0 and count.value == 1
+    leave_an_error_pending(L)
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(400_000_000)  # about 0.2 s
+    assert not stream.query()
+    assert L.pg_label_binary(ctypes.byref(dx), 2, ctypes.byref(do), ctypes.byref(count), s) != 0
+    assert stream.query()
