@@ -58,7 +58,6 @@ constexpr int kLabelIters = 1 << 24;
 constexpr int kLThreads = 256;
 constexpr int kLTile = 32 * kLThreads;             // pixels of a tile: one 32-pixel chunk of a row per thread
 constexpr int kLSegments = 2048;                   // most bitmap segments of the numbering pass
-constexpr int kLWords = 4 * kLThreads;             // bitmap words a numbering CTA scans at a time
 
 // which neighbours of the SE's raster-earlier half exist
 enum : unsigned { E_L = 1, E_U = 2, E_UL = 4, E_UR = 8, E_Z = 16 };
@@ -66,6 +65,7 @@ enum : unsigned { E_L = 1, E_U = 2, E_UL = 4, E_UR = 8, E_Z = 16 };
 struct LabelGeom {
   int64_t nx, ny, nz;
   int64_t tiles_x, tiles_y;  // tiles per slice
+  int slices;                // slices of a tile, one under the other (more than one only where tiles_y == 1)
   int64_t words_x;           // bitmap words per row (32 pixels each, rows padded)
   int log_tw;                // tile width (a multiple of 32); the height is kLTile >> log_tw
   unsigned edges;
@@ -131,7 +131,8 @@ template <typename T> __device__ __forceinline__ T shfl_up(T v, int d) {
   else return __shfl_up_sync(0xffffffffu, v, d);
 }
 
-template <typename T, bool FLAT>
+// STACKED: tiles of several slices.
+template <typename T, bool FLAT, bool STACKED>
 __global__ void __launch_bounds__(kLThreads) k_label_tile(const T *__restrict__ in, int32_t *__restrict__ par,
                                                           unsigned *__restrict__ roots, LabelGeom g) {
   // masks of the chunks: chunk id = chunk column * tile rows + row, so the chunk above is id - 1.
@@ -146,8 +147,10 @@ __global__ void __launch_bounds__(kLThreads) k_label_tile(const T *__restrict__ 
   const uint32_t tile = blockIdx.x, tiles_x = (uint32_t)g.tiles_x, tiles_y = (uint32_t)g.tiles_y;
   const int nx = (int)g.nx;  // the image has less than 2^31 pixels: its indices are 32-bit
   const int x0 = (int)(tile % tiles_x) << g.log_tw, y0 = (int)(tile / tiles_x % tiles_y) << log_th;
-  const int row0 = (int)(tile / tiles_x / tiles_y) * (int)g.ny + y0;  // first row, slices stacked
-  const int w = min(tw, nx - x0), h = min(th, (int)g.ny - y0);        // the tile inside the image
+  const int ny = (int)g.ny, z0 = (int)(tile / tiles_x / tiles_y) * (STACKED ? g.slices : 1);
+  const int row0 = z0 * ny + y0;  // first row, slices stacked
+  const int w = min(tw, nx - x0);  // the tile inside the image
+  const int h = STACKED ? min(g.slices, (int)g.nz - z0) * ny : min(th, ny - y0);
   const int base = row0 * nx + x0;
   const T *src = in + base;
   const bool hor = (g.edges & E_L) != 0, ver = (g.edges & E_U) != 0, eul = (g.edges & E_UL) != 0,
@@ -206,7 +209,8 @@ __global__ void __launch_bounds__(kLThreads) k_label_tile(const T *__restrict__ 
 
   // ---- runs: thread t owns chunk t
   const int id = threadIdx.x, r = id & (th - 1), cx = id >> log_th;
-  const bool has_left = cx > 0, has_right = (cx + 1) * 32 < tw, has_up = r > 0;  // neighbour chunks of the tile
+  const bool has_left = cx > 0, has_right = (cx + 1) * 32 < tw;      // neighbour chunks of the tile
+  const bool has_up = STACKED ? (unsigned)r % (unsigned)ny != 0u : r > 0;  // no edge up from a slice's first row
   const int l0 = (r << g.log_tw) + cx * 32;  // local raster index of the chunk's first pixel
   unsigned L, U = 0u, UL = 0u, UR = 0u, acc;
   {
@@ -259,6 +263,7 @@ __global__ void __launch_bounds__(kLThreads) k_label_tile(const T *__restrict__ 
     U &= ~(L & Ul & Lu);
     L &= 1u;  // inside a chunk the run holds it
   }
+  unsigned hang = 0u;  // runs that hang under another
   for (unsigned todo = starts; todo; todo &= todo - 1) {
     const unsigned bit = todo & (0u - todo), later = todo ^ bit;
     const unsigned run = ~(bit - 1) & (later ? (later & (0u - later)) - 1u : 0xffffffffu);
@@ -276,17 +281,17 @@ __global__ void __launch_bounds__(kLThreads) k_label_tile(const T *__restrict__ 
       to = run_of(id - th, 31);
     }
     s_p[ph(l)] = to;
+    if (to != l) hang |= bit;
   }
   __syncthreads();
   // pointer jumping: a link goes up a row or left a chunk, so six doublings flatten the usual tree
-  // (what is deeper still is walked by find_root)
+  // (what is deeper still is walked by find_root).  Roots stay where they are (in noise nearly every run is one).
   volatile int32_t *vp = s_p;
 #pragma unroll 1
   for (int it = 0; it < 6; ++it) {
-    for (unsigned todo = starts; todo; todo &= todo - 1) {
-      const int l = l0 + __ffs(todo) - 1;
-      const int32_t p = vp[ph(l)];
-      if (p != l) vp[ph(l)] = vp[ph(p)];
+    for (unsigned todo = hang; todo; todo &= todo - 1) {
+      const int i = ph(l0 + __ffs(todo) - 1);
+      vp[i] = vp[ph(vp[i])];
     }
     __syncthreads();
   }
@@ -424,12 +429,23 @@ __global__ void __launch_bounds__(kLThreads) k_label_flatten(int32_t *par, unsig
     if (m) {
       const int64_t row = (uint32_t)wi / (uint32_t)g.words_x;
       const int32_t i0 = (int32_t)(row * g.nx + (wi - row * g.words_x) * 32);
-      for (unsigned todo = m; todo; todo &= todo - 1) {
-        const int32_t i = i0 + __ffs(todo) - 1;
-        const int32_t p = __ldcg(par + i);
-        if (p == i) continue;
-        keep ^= todo & (0u - todo);
-        __stcg(par + i, find_root(par, p));
+      for (unsigned todo = m; todo;) {
+        // the loads of four roots go together (noise has nearly 32 a word: flat zones of 512^2 14 -> 6 us)
+        unsigned bit[4];
+        int32_t p[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          bit[k] = todo & (0u - todo);
+          todo ^= bit[k];
+          p[k] = bit[k] ? __ldcg(par + i0 + __ffs(bit[k]) - 1) : -1;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int32_t i = i0 + __ffs(bit[k]) - 1;
+          if (p[k] < 0 || p[k] == i) continue;
+          keep ^= bit[k];
+          __stcg(par + i, find_root(par, p[k]));
+        }
       }
       if (keep != m) roots[wi] = keep;
     }
@@ -442,7 +458,12 @@ __global__ void __launch_bounds__(kLThreads) k_label_flatten(int32_t *par, unsig
 }
 
 // CTA b numbers the roots of bitmap segment b: the roots before it are the sum of the earlier segments'
-// counts.  A root's parent word becomes -1 - number (numbers start at 1; -1 stays the background).
+// counts.  A root's parent word becomes -1 - number (numbers start at 1; -1 stays the background).  A thread scans
+// WPT words at a time: four, or one where the image is so small that four would leave most SMs without a segment.
+// A word with more than kLDense roots is written by its warp, a lane per pixel (whole lines), others by their thread.
+// (flat zones of 512^2 noise, nearly every pixel a root: 20 us with four words a thread and no whole lines, now 7).
+constexpr int kLDense = 16;
+template <int WPT>
 __global__ void __launch_bounds__(kLThreads) k_label_number(int32_t *__restrict__ par, const unsigned *__restrict__ roots,
                                                             const int32_t *__restrict__ cnt, LabelGeom g, int64_t words,
                                                             int log_seg, long long *__restrict__ total) {
@@ -464,12 +485,22 @@ __global__ void __launch_bounds__(kLThreads) k_label_number(int32_t *__restrict_
   if (cnt[blockIdx.x] == 0) return;
   const int64_t end = min(words, ((int64_t)blockIdx.x + 1) << log_seg);
   int buf = 1;
-  for (int64_t w0 = (int64_t)blockIdx.x << log_seg; w0 < end; w0 += kLWords, buf ^= 1) {
-    const int64_t wi = w0 + threadIdx.x * 4;  // four words per thread (the bitmap is padded to whole vectors)
-    uint4 m = make_uint4(0u, 0u, 0u, 0u);
-    if (wi < end) m = *reinterpret_cast<const uint4 *>(roots + wi);
-    const unsigned mw[4] = {m.x, wi + 1 < end ? m.y : 0u, wi + 2 < end ? m.z : 0u, wi + 3 < end ? m.w : 0u};
-    const int32_t own = __popc(mw[0]) + __popc(mw[1]) + __popc(mw[2]) + __popc(mw[3]);
+  for (int64_t w0 = (int64_t)blockIdx.x << log_seg; w0 < end; w0 += WPT * kLThreads, buf ^= 1) {
+    const int64_t wi = w0 + threadIdx.x * WPT;
+    unsigned mw[WPT];
+    if constexpr (WPT == 4) {  // the bitmap is padded to whole vectors
+      uint4 m = make_uint4(0u, 0u, 0u, 0u);
+      if (wi < end) m = *reinterpret_cast<const uint4 *>(roots + wi);
+      mw[0] = m.x;
+      mw[1] = wi + 1 < end ? m.y : 0u;
+      mw[2] = wi + 2 < end ? m.z : 0u;
+      mw[3] = wi + 3 < end ? m.w : 0u;
+    } else {
+      mw[0] = wi < end ? roots[wi] : 0u;
+    }
+    int32_t own = 0;
+#pragma unroll
+    for (int j = 0; j < WPT; ++j) own += __popc(mw[j]);
     int32_t incl = own;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -487,11 +518,20 @@ __global__ void __launch_bounds__(kLThreads) k_label_number(int32_t *__restrict_
     }
     int32_t code = -1 - (base + pre + incl - own);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (!mw[j]) continue;
+    for (int j = 0; j < WPT; ++j) {
+      const unsigned m = mw[j];
       const int64_t row = (uint32_t)(wi + j) / (uint32_t)g.words_x;
-      const int64_t i0 = row * g.nx + (wi + j - row * g.words_x) * 32;
-      for (unsigned todo = mw[j]; todo; todo &= todo - 1) par[i0 + __ffs(todo) - 1] = --code;
+      const int32_t i0 = (int32_t)(row * g.nx + (wi + j - row * g.words_x) * 32);
+      const bool dense = __popc(m) > kLDense;
+      for (unsigned todo = __ballot_sync(0xffffffffu, dense); todo; todo &= todo - 1) {
+        const int w = __ffs(todo) - 1;
+        const unsigned mo = __shfl_sync(0xffffffffu, m, w);
+        const int32_t first = __shfl_sync(0xffffffffu, i0, w), c = __shfl_sync(0xffffffffu, code, w);
+        if ((mo >> lane) & 1u) par[first + lane] = c - 1 - __popc(mo & ((1u << lane) - 1u));
+      }
+      if (dense) code -= __popc(m);
+      else
+        for (unsigned todo = m; todo; todo &= todo - 1) par[i0 + __ffs(todo) - 1] = --code;
     }
     base += all;
   }
@@ -538,24 +578,41 @@ bool upper_edges(int se, unsigned *e) {
 
 template <typename T, bool FLAT>
 pg_status label_t(const pg_image &in, const pg_image &out, unsigned edges, int64_t *count, cudaStream_t s) {
-  const Dims d = dims_of(in);
+  Dims d = dims_of(in);
   const int64_t n = d.count();
+  // Axes of length 1 are dropped, so that what is left lies along rows: a column is a row whose edges up are edges
+  // left (300000 pixels: 78 us as a column, 57 as a row)
+  if (d.nx == 1) {
+    edges = (edges & E_U ? E_L : 0u) | (edges & E_Z ? E_U : 0u);
+    d.nx = d.ny; d.ny = d.nz; d.nz = 1;
+  }
+  if (d.ny == 1 && d.nz > 1) {
+    edges = (edges & E_L) | (edges & E_Z ? E_U : 0u);
+    d.ny = d.nz; d.nz = 1;
+  }
+  if (d.nx == 1) {  // only the slices were many
+    edges = edges & E_U ? E_L : 0u;
+    d.nx = d.ny; d.ny = 1;
+  }
   LabelGeom g{};
   g.nx = d.nx; g.ny = d.ny; g.nz = d.nz;
   g.edges = edges;
-  // tiles of 128 x 64 pixels (1 pixel in 43 on a border); images of a few rows take wider ones, so
-  // that a tile is not mostly outside
-  g.log_tw = 7;
-  while (g.log_tw < 13 && (kLTile >> g.log_tw) / 2 >= d.ny) ++g.log_tw;
+  // Tiles of 128 x 64 pixels (1 pixel in 43 on a border).  So that a tile is not mostly outside the image, images of
+  // up to 32 columns take 32 x 256, images of a few rows wider ones, and a tile holds as many slices of a volume as
+  // fit (a tile 128 pixels wide per slice: 20000 binary slices of 8 x 8 333 us, now 89; 60000 x 32 flat 81, now 63).
+  g.log_tw = d.nx <= 32 ? 5 : 7;
+  while (g.log_tw < 13 && (kLTile >> g.log_tw) / 2 >= d.ny * d.nz) ++g.log_tw;
   const int64_t tw = 1ll << g.log_tw, th = kLTile >> g.log_tw;
   g.tiles_x = ceil_div(d.nx, tw);
   g.tiles_y = ceil_div(d.ny, th);
+  // (one slice a tile while that gives no more than two tiles an SM: 64^3 62 us, 72 with two slices)
+  g.slices = g.tiles_x * g.tiles_y * d.nz <= 2 * num_sms() ? 1 : (int)std::max<int64_t>(std::min(th / d.ny, d.nz), 1);
   g.words_x = ceil_div(d.nx, 32);
-  const int64_t words = g.words_x * d.ny * d.nz, tiles = g.tiles_x * g.tiles_y * d.nz;
-  // bitmap segments: whole chunks of the numbering pass, kLSegments of them at most (a segment's CTA
-  // sums the counts before it)
-  int log_seg = 10;
-  static_assert(kLWords == 1 << 10, "a segment holds whole chunks");
+  const int64_t words = g.words_x * d.ny * d.nz, tiles = g.tiles_x * g.tiles_y * ceil_div(d.nz, (int64_t)g.slices);
+  // bitmap segments: whole chunks of the numbering pass (kLThreads words of one or four a thread), kLSegments of them
+  // at most (a segment's CTA sums the counts before it)
+  static_assert(kLThreads == 1 << 8, "a segment holds whole chunks");
+  int log_seg = ceil_div(words, kLThreads) <= 4 * num_sms() ? 8 : 10;
   while (ceil_div(words, 1ll << log_seg) > kLSegments) ++log_seg;
   const int64_t nseg = ceil_div(words, 1ll << log_seg);
   const size_t par_bytes = (sizeof(int32_t) * (size_t)n + 255) / 256 * 256;
@@ -572,7 +629,8 @@ pg_status label_t(const pg_image &in, const pg_image &out, unsigned edges, int64
   int64_t *o = static_cast<int64_t *>(out.data);
   const T *src = static_cast<const T *>(in.data);
   PG_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)nseg, s), "clear label counts");
-  k_label_tile<T, FLAT><<<(unsigned)tiles, kLThreads, 0, s>>>(src, par, roots, g);
+  if (g.slices > 1) k_label_tile<T, FLAT, true><<<(unsigned)tiles, kLThreads, 0, s>>>(src, par, roots, g);
+  else k_label_tile<T, FLAT, false><<<(unsigned)tiles, kLThreads, 0, s>>>(src, par, roots, g);
   const int64_t n_rows = (edges & (E_U | E_UL | E_UR)) ? d.nz * (g.tiles_y - 1) * d.nx : 0;
   const int64_t n_cols = (edges & (E_L | E_UL | E_UR)) ? d.nz * d.ny * (g.tiles_x - 1) : 0;
   const int64_t n_z = (edges & E_Z) ? (d.nz - 1) * d.ny * d.nx : 0;
@@ -581,7 +639,8 @@ pg_status label_t(const pg_image &in, const pg_image &out, unsigned edges, int64
     k_label_border<T, FLAT><<<(unsigned)std::min<int64_t>(ceil_div(items, kLThreads), cap), kLThreads, 0, s>>>(
         src, par, g, n_rows, n_cols, n_z);
   k_label_flatten<<<(unsigned)ceil_div(words, kLThreads), kLThreads, 0, s>>>(par, roots, cnt, g, words, log_seg);
-  k_label_number<<<(unsigned)nseg, kLThreads, 0, s>>>(par, roots, cnt, g, words, log_seg, total);
+  if (log_seg < 10) k_label_number<1><<<(unsigned)nseg, kLThreads, 0, s>>>(par, roots, cnt, g, words, log_seg, total);
+  else k_label_number<4><<<(unsigned)nseg, kLThreads, 0, s>>>(par, roots, cnt, g, words, log_seg, total);
   const unsigned rg = (unsigned)ceil_div(n, 4 * kLThreads);
   if (reinterpret_cast<uintptr_t>(o) % 16 == 0) k_label_resolve<true><<<rg, kLThreads, 0, s>>>(par, n, o);
   else k_label_resolve<false><<<rg, kLThreads, 0, s>>>(par, n, o);
