@@ -510,8 +510,49 @@ __global__ void __launch_bounds__(kWThreads, sizeof(T) == 1 ? 3 : 4) k_chords(co
   }
 }
 
+// How an image is cut for k_chords.
+struct ChordTiles {
+  int vw;            // output words of a tile row, as in window_t
+  int tiles_x;
+  int rows;          // R, the rows a thread holds: half a tile's
+  int64_t tiles;
+};
+// R is what three (u8, two registers a row) or four CTAs per SM leave room for (2048^2 u8, radius 5: 12 rows 29 us,
+// 16 rows 35, 8 rows 34; f32: 16 rows 49, 12 rows 51, 8 rows 60); 4 where the image would not give every SM a tile.
+constexpr int chord_rows(int es) { return es == 1 ? 12 : 16; }
+ChordTiles chord_tiles(const pg_image &in, const pg_image &out, int max_len) {
+  const int es = elem_size(in.ptype), E = 4 / es;
+  const Dims d = dims_of(in);
+  ChordTiles c{};
+  c.vw = std::min((kWRow * E - (max_len - 1)) / E - 2, kWOut) & ~7;
+  const bool mis = E > 1 && (d.nx % E != 0 || reinterpret_cast<uintptr_t>(out.data) % 4 != 0);
+  c.tiles_x = (int)ceil_div(d.nx + (mis ? E - 1 : 0), (int64_t)c.vw * E);
+  c.rows = chord_rows(es);
+  if (c.tiles_x * ceil_div(d.ny, 2 * c.rows) * d.nz < num_sms()) c.rows = 4;
+  c.tiles = c.tiles_x * ceil_div(d.ny, 2 * c.rows) * d.nz;
+  return c;
+}
+
+// Whether the chords beat the gather of small_se.cu on this image, by the times of both in nanoseconds (fitted to
+// 3200 lists and images, 6 % and 20 % off: the slower one by more than 8 % is taken on 64 of them).  A gather costs its loads; the groups of a tile go one after the other,
+// which is what a small image waits for (61 offsets of two diagonals on 64^2 u8: 48 us, gathered 15), and a tile
+// that an image fills only in part costs as much as a full one (a disk of 5 offsets on 200000 x 2 u8: 144 us, 11).
+bool chords_win(const ChordTable &t, const ChordTiles &c, const Dims &d, int es, int n) {
+  const double pixels = (double)d.count(), th = 2 * c.rows;
+  double wait = 4200., rows = 0., adds = 0.;
+  for (int k = 0; k < t.n; ++k) {
+    const double r = th + t.g[k].dy_max - t.g[k].dy_min;  // rows of windows a tile makes, 16 at a time
+    wait += 550. + 650. * (double)ceil_div((int64_t)r, 2 * kWWarps);
+    rows += r;
+    adds += t.g[k].count * th;
+  }
+  const double chords = wait + (double)c.tiles * (0.12 * rows + (es == 1 ? 0.028 : 0.014) * adds + 4.);
+  const double gather = 6500. + 105. * n + 0.001 * (n + 4) * pixels;
+  return chords < gather;
+}
+
 template <typename T, bool SUP, int R>
-pg_status chords_r(const pg_image &in, const pg_image &out, const ChordTable &t, int vw, int tiles_x, int span,
+pg_status chords_r(const pg_image &in, const pg_image &out, const ChordTable &t, const ChordTiles &c, int span,
                    cudaStream_t s) {
   const Dims d = dims_of(in);
   static std::atomic<uint64_t> attr_devices{0};
@@ -523,25 +564,16 @@ pg_status chords_r(const pg_image &in, const pg_image &out, const ChordTable &t,
                 "neighbour-list kernel smem attribute");
     attr_devices.fetch_or(bit);
   }
-  const dim3 grid((unsigned)tiles_x, (unsigned)ceil_div(d.ny, 2 * R), (unsigned)d.nz);
+  const dim3 grid((unsigned)c.tiles_x, (unsigned)ceil_div(d.ny, 2 * R), (unsigned)d.nz);
   k_chords<T, SUP, R><<<grid, kWThreads, (size_t)(2 * R + span) * kWRow * 4, s>>>(
-      static_cast<const T *>(in.data), static_cast<T *>(out.data), d.nz, d.ny, d.nx, vw, t);
+      static_cast<const T *>(in.data), static_cast<T *>(out.data), d.nz, d.ny, d.nx, c.vw, t);
   return cuda_status(cudaGetLastError(), "neighbour-list kernel launch");
 }
 
 template <typename T, bool SUP>
-pg_status chords_t(const pg_image &in, const pg_image &out, const ChordTable &t, int max_len, int span, cudaStream_t s) {
-  constexpr int E = 4 / (int)sizeof(T);
-  const Dims d = dims_of(in);
-  const int vw = std::min((kWRow * E - (max_len - 1)) / E - 2, kWOut) & ~7;  // as in window_t
-  const bool mis = E > 1 && (d.nx % E != 0 || reinterpret_cast<uintptr_t>(out.data) % 4 != 0);
-  const int tiles_x = (int)ceil_div(d.nx + (mis ? E - 1 : 0), (int64_t)vw * E);
-  // Rows a thread holds, half a tile's: what three (u8, two registers a row) or four CTAs per SM leave room for
-  // (2048^2 u8, radius 5: 12 rows 29 us, 16 rows 35, 8 rows 34; f32: 16 rows 49, 12 rows 51, 8 rows 60); 4
-  // where the image would not give every SM a tile.
-  constexpr int R = sizeof(T) == 1 ? 12 : 16;
-  if (tiles_x * ceil_div(d.ny, 2 * R) * d.nz < num_sms()) return chords_r<T, SUP, 4>(in, out, t, vw, tiles_x, span, s);
-  return chords_r<T, SUP, R>(in, out, t, vw, tiles_x, span, s);
+pg_status chords_t(const pg_image &in, const pg_image &out, const ChordTable &t, const ChordTiles &c, int span, cudaStream_t s) {
+  constexpr int R = chord_rows((int)sizeof(T));
+  return c.rows == R ? chords_r<T, SUP, R>(in, out, t, c, span, s) : chords_r<T, SUP, 4>(in, out, t, c, span, s);
 }
 
 // The list as chords; false where it has too many, or where they are so short that gathering the offsets one
@@ -640,11 +672,13 @@ bool try_chords(const pg_image &in, const pg_image &out, const int32_t *offsets,
   ChordTable t;
   int span = 0, longest = 1;
   if (!make_chords(offsets, n, in.rank, 4 / es, es == 4 ? 32 : 64, t, span, longest)) return false;
+  const ChordTiles c = chord_tiles(in, out, longest);
+  if (!chords_win(t, c, d, es, n)) return false;
   switch (in.ptype) {
-    case PG_PTYPE_U8: *st = dilate ? chords_t<uint8_t, true>(in, out, t, longest, span, s) : chords_t<uint8_t, false>(in, out, t, longest, span, s); return true;
-    case PG_PTYPE_U16: *st = dilate ? chords_t<uint16_t, true>(in, out, t, longest, span, s) : chords_t<uint16_t, false>(in, out, t, longest, span, s); return true;
-    case PG_PTYPE_I32: *st = dilate ? chords_t<int32_t, true>(in, out, t, longest, span, s) : chords_t<int32_t, false>(in, out, t, longest, span, s); return true;
-    case PG_PTYPE_F32: *st = dilate ? chords_t<float, true>(in, out, t, longest, span, s) : chords_t<float, false>(in, out, t, longest, span, s); return true;
+    case PG_PTYPE_U8: *st = dilate ? chords_t<uint8_t, true>(in, out, t, c, span, s) : chords_t<uint8_t, false>(in, out, t, c, span, s); return true;
+    case PG_PTYPE_U16: *st = dilate ? chords_t<uint16_t, true>(in, out, t, c, span, s) : chords_t<uint16_t, false>(in, out, t, c, span, s); return true;
+    case PG_PTYPE_I32: *st = dilate ? chords_t<int32_t, true>(in, out, t, c, span, s) : chords_t<int32_t, false>(in, out, t, c, span, s); return true;
+    case PG_PTYPE_F32: *st = dilate ? chords_t<float, true>(in, out, t, c, span, s) : chords_t<float, false>(in, out, t, c, span, s); return true;
     default: return false;
   }
 }
