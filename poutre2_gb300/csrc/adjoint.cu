@@ -596,7 +596,15 @@ __global__ void __launch_bounds__(AS_THREADS) k_flat_bwd_arg_strip(const unsigne
 }
 
 // Whether the strip kernels take these planes, and their geometry.
-static bool strip_geom(const void *a, const void *b, const void *code, int64_t planes, int64_t h, int64_t w, StripGeom &g) {
+// They do where there are units enough to fill the GPU and the strips' work -- pixels walked, with the 2r rows beside
+// a strip and the columns past the last segment -- is not much more than that of the shared-memory tiles above
+// (2500 shapes up to 40 Mpixel drawn, us, strips / tiles).  Forward: a pass of fewer units waits for one strip's chain
+// of rows (1 x 256 x 256, r = 2: 6.3 / 4.3; 256 x 64 x 64 6.6 / 8.6), narrow rows leave lanes idle (256 x 200 x 4 12.7 / 10.6).
+// Backward: r = 1 wins nearly always, r = 2 as the forward (1 x 1024 x 1024 12.5 / 10.3), r = 3 is so much arithmetic
+// that only long strips of full segments win, or where the tiles are half empty (2048 x 256 x 256 690 / 764, 2048 x 240 x
+// 240 slower, 1676 x 64 x 128 123 / 111, 517 x 159 x 64 54 / 82).
+static bool strip_geom(const void *a, const void *b, const void *code, int64_t planes, int64_t h, int64_t w, int r,
+                       bool backward, StripGeom &g) {
   if (w % 4 != 0 || (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % 16 != 0 ||
       reinterpret_cast<uintptr_t>(code) % 4 != 0)
     return false;
@@ -611,7 +619,19 @@ static bool strip_geom(const void *a, const void *b, const void *code, int64_t p
   g.strips = (int)ceil_div(h, g.strip);
   g.strip = (int)ceil_div(h, g.strips);  // evenly
   g.units = planes * g.strips * g.segs;
-  return ceil_div(g.units * AS_LANES, AS_THREADS) <= INT32_MAX;
+  if (ceil_div(g.units * AS_LANES, AS_THREADS) > INT32_MAX) return false;
+  const int wx = 2 * r + 1, sms = num_sms();
+  const double walked = (double)g.units * AS_COLS * (double)(ceil_div(g.strip + 2 * r, wx) * wx);
+  if (!backward || r == 2) {
+    const int tile_w = backward ? 4 * AQ_QUADS : AF_TX - 2 * r;
+    const double tiles = (double)planes * (double)(ceil_div(h, AT_H) * AT_H) * (double)(ceil_div(w, tile_w) * tile_w);
+    if (backward) return g.units >= 13 * sms && 0.8 * walked <= tiles;
+    return r == 1 ? g.units >= 9 * sms || (g.units >= 3 * sms && 2. * walked <= tiles) : g.units >= 6 * sms && 0.7 * walked <= tiles;
+  }
+  if (r == 1) return h > AT_H / 2 || g.units >= 4 * sms;
+  // a tile's warps without columns in the image, and its rows below it, cost nothing here
+  return (int64_t)g.segs * AS_COLS * 20 <= w * 21 && g.units >= 6 * sms &&
+         0.8 * walked <= (double)planes * (double)h * (double)(ceil_div(w, 128) * 128);
 }
 
 template <bool SUP>
@@ -888,7 +908,7 @@ pg_status launch_flat2d_arg(const float *x, float *y, unsigned char *code, int64
   if (h > (1 << 30) || w > (1 << 30) || ceil_div(h, AT_H) > 65535 || planes > 65535)
     return fail(PG_ERR_INVALID_ARGUMENT, "plane too large");
   StripGeom g;
-  if (strip_geom(x, y, code, planes, h, w, g)) {
+  if (strip_geom(x, y, code, planes, h, w, r, false, g)) {
     const unsigned ctas = (unsigned)ceil_div(g.units * AS_LANES, AS_THREADS);
     if (dilate) {
       if (r == 1) k_flat_fwd_arg_strip<true, 1><<<ctas, AS_THREADS, 0, s>>>(x, y, code, g);
@@ -921,10 +941,8 @@ pg_status launch_flat2d_backward_arg(const unsigned char *code, const float *gy,
   if (planes * h * w == 0) return PG_OK;
   if (h > (1 << 30) || w > (1 << 30) || ceil_div(h, AT_H) > 65535 || planes > 65535)
     return fail(PG_ERR_INVALID_ARGUMENT, "plane too large");
-  // The 7x7 backward is so much arithmetic that the strips only win where their segments are nearly full: 256
-  // columns 690 us against 764, 320 176 / 224, but 240 102 / 98 and 160 slower still.
   StripGeom g;
-  if (strip_geom(gy, gx, code, planes, h, w, g) && (r < 3 || (int64_t)g.segs * AS_COLS * 20 <= w * 21)) {
+  if (strip_geom(gy, gx, code, planes, h, w, r, true, g)) {
     const unsigned ctas = (unsigned)ceil_div(g.units * AS_LANES, AS_THREADS);
     if (r == 1) k_flat_bwd_arg_strip<1><<<ctas, AS_THREADS, 0, s>>>(code, gy, gx, g);
     else if (r == 2) k_flat_bwd_arg_strip<2><<<ctas, AS_THREADS, 0, s>>>(code, gy, gx, g);
