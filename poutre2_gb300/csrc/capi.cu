@@ -183,18 +183,17 @@ static pg_status repeat_small(const pg_image &in, int se, int iter, const pg_ima
 static pg_status box(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, bool dilate, cudaStream_t s) {
   const int es = elem_size(in.ptype);
   const bool words = rows_aligned(in, out, 4), vectors = rows_aligned(in, out, 16);
-  const bool window = window_ok(in, out, hy, hx, 0);
   pg_status st = PG_OK;
   const int64_t n = dims_of(in).count();
-  if (hx == 1 && hy <= 1 && !vectors && window && n >= (es <= 2 ? 3 << 20 : 8 << 20) &&
-      try_window(in, out, hy, hx, 0, dilate, s, &st))
+  if (hx == 1 && hy <= 1 && !vectors && n >= (es <= 2 ? 3 << 20 : 8 << 20) && try_window(in, out, hy, hx, 0, dilate, s, &st))
     return st;
   if (hy == 0 && hx == 1)
     return launch_small_se(in, out, in.rank == 1 ? PG_SE_SEGMENT_X_1D : PG_SE_SEGMENT_X_2D, dilate, s);
   if (in.rank == 2 && hy == 1 && hx == 0) return launch_small_se(in, out, PG_SE_SEGMENT_Y_2D, dilate, s);
-  const int64_t square_passes_max =
-      window ? (vectors && n >= (4 << 20) ? 2 : 1) : (es <= 2 ? 4 : 2);
-  if (in.rank == 2 && hy == hx && hy >= 1 && hy <= square_passes_max)
+  if (in.rank == 2 && hy == 1 && hx == 1) return launch_small_se(in, out, PG_SE_SQUARE_2D, dilate, s);
+  const bool window = window_ok(in, out, hy, hx, 0);
+  const int64_t square_passes_max = window ? (vectors && n >= (4 << 20) ? 2 : 1) : (es <= 2 ? 4 : 2);
+  if (in.rank == 2 && hy == hx && hy >= 2 && hy <= square_passes_max)
     return repeat_small(in, PG_SE_SQUARE_2D, (int)hy, out, dilate, s);
   // Y segment: the segment tile kernel (diag.cu), measured faster than the box tile for every type
   if (hx == 0 && hy <= 31 && try_segment_tile(in, out, 1, 0, (int)hy, dilate, s, &st)) return st;

@@ -194,15 +194,20 @@ pg_status launch_line(const pg_image &in, const pg_image &out, int dy, int dx, i
   const int64_t k = std::min<int64_t>(half, std::max<int64_t>(kmax, 0));
   if (k >= 1 && k <= (1 << 20)) {
     // Y and diagonal segments: the TMA tiles or the register streams where they have the length, else the
-    // window kernel (4096^2, us, with / without it: u8 Y k = 10 25 / 24, 8192^2 57 / 72; f32 Y k = 10 45 / 61;
-    // u8 45 degrees k = 10 26 / 45, f32 43 / 104; ragged 2999 x 4001 u8 Y 22 / 68, 45 degrees 21 / 90).  Long Y
-    // segments of small images keep the word tiles of line_w.cu where rows are whole words: their tiles are
-    // narrow, and a small image gives the window kernel few (u16 3380 x 558, k = 28: 18 / 10).
+    // window kernel (4096^2, us, with / without it: u8 45 degrees k = 10 26 / 45, f32 43 / 104; ragged 2999 x 4001 u8 Y
+    // 22 / 68, 45 degrees 21 / 90).  Y segments of whole-word rows keep the word tiles of line_w.cu where those are the
+    // faster: u8 between 1.5 and 20 Mpixel (k = 4 to 30: 3735 x 7360 23 / 27, 1975 x 628 8 / 9, but 1520 x 5856 21 / 15, 903 x
+    // 2900 11 / 9; from k = 36 on up to 7: 5190 x 3584 k = 60 44 / 54) and long ones of small images (k above 10; u16
+    // 912 x 12400 21 / 25 but 3029 x 1488 15 / 11, f32 854 x 6848 20 / 23).
     pg_status st = PG_OK;
     if (dx != 0 && try_segment_tile(in, out, dy, dx, (int)k, dilate, s, &st)) return st;
     if (try_line_stream(in, out, dy, dx, (int)k, dilate, s, &st)) return st;
     const bool words = rows_aligned(in, out, 4);
-    if (dx == 0 && (!words || k <= 10 || d.count() >= (4 << 20)) && try_window(in, out, k, 0, 0, dilate, s, &st)) return st;
+    const int es = elem_size(in.ptype);
+    const int64_t n = d.count();
+    const int64_t big = (es == 4 ? 4 : es == 2 ? 8 : k >= 36 ? 7 : 20) << 20;
+    const bool window_y = !words || n >= big || (k <= 10 && (es != 1 || n < (3 << 19)));
+    if (dx == 0 && window_y && try_window(in, out, k, 0, 0, dilate, s, &st)) return st;
     if (dx != 0 && dy != 0 && try_window(in, out, k, 0, dx, dilate, s, &st)) return st;
     if (dy == 0 && !words && try_window(in, out, 0, k, 0, dilate, s, &st)) return st;
     if (try_line_words(in, out, dy, dx, (int)k, dilate, s, &st)) return st;

@@ -150,6 +150,8 @@ struct WindowGeom {
   int half;        // half the rows of the tile's array in shared memory, a multiple of 6
   int vw;          // output words of a tile row
   int64_t u_first; // first pixel of tile column 0 at the tile's first output row
+  int64_t tiles_x, tiles_y;
+  double work;     // 64-row tiles of a 3-row window per SM that this costs
 };
 
 // Columns, in place: word of row i <- op over rows [i, i + N), N = 3 or 9 (the min / max of three values is
@@ -414,9 +416,17 @@ __global__ void __launch_bounds__(kWThreads) k_window(const T *__restrict__ in, 
   }
 }
 
-template <typename T, bool SUP>
-pg_status window_t(const pg_image &in, const pg_image &out, WindowGeom g, cudaStream_t s) {
-  constexpr int E = 4 / (int)sizeof(T);
+WindowGeom window_geom(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, int lean) {
+  const int E = 4 / elem_size(in.ptype);
+  const Dims d = dims_of(in);
+  WindowGeom g{};
+  g.H = d.ny;
+  g.W = d.nx;
+  // clipped windows reach no further than the image: on one column (row) they are the pixels themselves, with no
+  // neutral value beside them to stand in for an infinity
+  g.hx = (int)std::min(hx, d.nx - 1);
+  g.hy = (int)std::min(hy, d.ny - 1);
+  g.lean = lean;
   // valid words of a row (windows are forward), in whole 32-byte sectors: a misaligned load loses a word, the
   // stores' shift needs one left of the tile
   g.vw = std::min((kWRow * E - 2 * g.hx) / E - 2, kWOut) & ~7;
@@ -429,8 +439,16 @@ pg_status window_t(const pg_image &in, const pg_image &out, WindowGeom g, cudaSt
   auto tiles_x = [&]() { return ceil_div(g.W + (g.lean ? g.th - 1 : 0) + (mis ? E - 1 : 0), (int64_t)g.vw * E); };
   while (g.th > 16 && g.th / 2 >= 2 * g.hy && tiles_x() * ceil_div(g.H, g.th) < 4 * sms) g.th /= 2;
   if (tiles_x() * ceil_div(g.H, g.th) < sms) g.th /= 2;  // 64, 32, 16 or 8: a group's rows are a multiple of 4
+  g.tiles_x = tiles_x();
+  g.tiles_y = ceil_div(g.H, g.th);
+  g.work = (double)(g.tiles_x * g.tiles_y) * (g.th + 2 * g.hy) / (66. * (double)sms);
   g.u_first = g.lean > 0 ? -(int64_t)(g.th - 1) : 0;
   g.half = (g.th + 2 * g.hy + 11) / 12 * 6;
+  return g;
+}
+
+template <typename T, bool SUP>
+pg_status window_t(const pg_image &in, const pg_image &out, const WindowGeom &g, cudaStream_t s) {
   const size_t smem = (size_t)(2 * g.half) * kWRow * 4;
   static std::atomic<uint64_t> attr_devices{0};
   int dev = 0;
@@ -441,7 +459,7 @@ pg_status window_t(const pg_image &in, const pg_image &out, WindowGeom g, cudaSt
                 "window kernel smem attribute");
     attr_devices.fetch_or(bit);
   }
-  const dim3 grid((unsigned)tiles_x(), (unsigned)ceil_div(g.H, g.th));
+  const dim3 grid((unsigned)g.tiles_x, (unsigned)g.tiles_y);
   k_window<T, SUP><<<grid, kWThreads, smem, s>>>(static_cast<const T *>(in.data), static_cast<T *>(out.data), g);
   return cuda_status(cudaGetLastError(), "window kernel launch");
 }
@@ -626,6 +644,26 @@ bool make_chords(const int32_t *offsets, int n, int rank, int pixels_per_word, i
   return 50 * t.n + 5 * nc <= 14 * n * pixels_per_word;
 }
 
+// A tile costs the same however little of its rows the image fills: where narrow images give the GPU more work than
+// it has room for at once, the kernels that work in columns or narrow tiles are faster (us, window / other):
+//   rectangles on whole-word rows of 1- and 2-byte pixels, and repeated 3x3 squares: u8 100000 x 8 5x5 58 / 13, 30000 x 64
+//     21x21 31 / 24, u16 168033 x 5 5x5 78 / 15, but u8 1239 x 48 5x7 7 / 17, u16 11063 x 96 3x51 11 / 22;
+//   vertical segments: whole-word rows up to 640 bytes (f32 k = 9 30068 x 144 25 / 21, 81041 x 128 54 / 35, 11734 x 338
+//     17 / 18); ragged ones of a few pixels (u8 48833 x 21 k = 39 52 / 36, but 8461 x 18 k = 6 13 / 29);
+//   45 / 135 degrees: u16 18835 x 6 k = 5 17 / 13;
+//   one column: a row segment is a copy (u8 194408 x 1 115 / 4); others u8 182485 x 1 5 x 117 129 / 62.
+bool window_narrow(const WindowGeom &g, int64_t hy, int64_t hx, int es, bool words) {
+  const int64_t row = g.W * es;
+  const double work = g.work;
+  if (g.W == 1) return (g.hy == 0 && g.hx == 0) || work >= 4.;
+  if (g.lean != 0) return words && es <= 2 && ((row <= 16 && work >= 3.) || (row <= 48 && work >= 8.));
+  if (hx == 0) return words ? (row <= 640 && work >= 3.) || (row <= 48 && work >= 1.) : row <= 24 && work >= 5.;
+  const bool squares = hy == hx && hy <= (es <= 2 ? 4 : 2);
+  if (squares || (hx == 1 && hy <= 1)) return row <= 256 && work >= 4.;
+  if (hy == 0 || es > 2 || !words) return false;
+  return (row <= 256 && work >= 4.5) || (es == 1 && row <= 32 && work >= 1.2);
+}
+
 }  // namespace
 
 bool window_ok(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, int lean) {
@@ -637,21 +675,14 @@ bool window_ok(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, 
   const Dims d = dims_of(in);
   if (d.ny < 16 || d.nx < 1 || d.ny > (1 << 19) || d.nx > (1 << 30)) return false;
   const uintptr_t pixel = (uintptr_t)es - 1;
-  return ((reinterpret_cast<uintptr_t>(in.data) | reinterpret_cast<uintptr_t>(out.data)) & pixel) == 0;
+  if (((reinterpret_cast<uintptr_t>(in.data) | reinterpret_cast<uintptr_t>(out.data)) & pixel) != 0) return false;
+  return !window_narrow(window_geom(in, out, hy, hx, lean), hy, hx, es, rows_aligned(in, out, 4));
 }
 
 bool try_window(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx, int lean, bool dilate, cudaStream_t s,
                 pg_status *st) {
   if (!window_ok(in, out, hy, hx, lean)) return false;
-  const Dims d = dims_of(in);
-  WindowGeom g{};
-  g.H = d.ny;
-  g.W = d.nx;
-  // clipped windows reach no further than the image: on one column (row) they are the pixels themselves, with no
-  // neutral value beside them to stand in for an infinity
-  g.hx = (int)std::min(hx, d.nx - 1);
-  g.hy = (int)std::min(hy, d.ny - 1);
-  g.lean = lean;
+  const WindowGeom g = window_geom(in, out, hy, hx, lean);
   switch (in.ptype) {
     case PG_PTYPE_U8: *st = dilate ? window_t<uint8_t, true>(in, out, g, s) : window_t<uint8_t, false>(in, out, g, s); return true;
     case PG_PTYPE_U16: *st = dilate ? window_t<uint16_t, true>(in, out, g, s) : window_t<uint16_t, false>(in, out, g, s); return true;
