@@ -38,7 +38,14 @@ def leave_an_error_pending(L):
 
 
 def capped_reconstruction(L):
-    """Queues a reconstruction that gives up after one visit a tile."""
+    """A reconstruction that gave up after one visit a tile."""
+    s = capped_reconstruction_on(L, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    return s
+
+
+def capped_reconstruction_on(L, stream):
+    """Queues it on `stream` and waits for it there."""
     from poutre2_gb300.image import descriptor
     f = np.zeros((256, 256), np.uint8)
     f[::4] = 100
@@ -48,12 +55,13 @@ def capped_reconstruction(L):
     m[0, 0] = 100
     k, mk = torch.from_numpy(f).cuda(), torch.from_numpy(m).cuda()
     out = torch.empty_like(k)
-    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    torch.cuda.current_stream().synchronize()
+    s = ctypes.c_void_p(stream.cuda_stream)
     d = [descriptor(x) for x in (mk, k, out)]
     assert L.pg_debug_set_limits(1, 0) == 0
     assert L.pg_reconstruction(1, ctypes.byref(d[0]), ctypes.byref(d[1]), 2, ctypes.byref(d[2]), s) == 0
     assert L.pg_debug_set_limits(0, 0) == 0
-    torch.cuda.synchronize()
+    stream.synchronize()
     return s
 
 
@@ -82,3 +90,43 @@ def test_a_failed_labelling_keeps_its_word_until_its_kernels_ended(L):
     assert not stream.query()
     assert L.pg_label_binary(ctypes.byref(dx), 2, ctypes.byref(do), ctypes.byref(count), s) != 0
     assert stream.query()
+
+
+def test_more_calls_than_pinned_words(L):
+    # 64 labellings behind a long kernel hold every word: the next count and the next status come by copies
+    import threading
+
+    from poutre2_gb300.image import descriptor
+    n = 64
+    busy, free = torch.cuda.Stream(), torch.cuda.Stream()
+    x = torch.zeros(40, 70, dtype=torch.uint8, device="cuda")
+    x[::3, ::4] = 1  # 14 x 18 pixels of their own
+    outs = [torch.empty(40, 70, dtype=torch.int64, device="cuda") for _ in range(n + 1)]
+    counts, statuses = [ctypes.c_int64(-1) for _ in range(n + 1)], [None] * (n + 1)
+    dx, ds = descriptor(x), [descriptor(o) for o in outs]
+    capped_reconstruction(L)
+    L.pg_check_device(ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+
+    def label(i):
+        s = ctypes.c_void_p((busy if i < n else free).cuda_stream)
+        statuses[i] = L.pg_label_binary(ctypes.byref(dx), 3, ctypes.byref(ds[i]), ctypes.byref(counts[i]), s)
+
+    label(n)
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(2_000_000_000)  # about a second
+    threads = [threading.Thread(target=label, args=(i,)) for i in range(n)]
+    for t in threads:
+        t.start()
+    import time
+    time.sleep(0.2)  # every thread is in its call
+    counts[n].value = -1
+    label(n)
+    s = capped_reconstruction_on(L, free)
+    status = L.pg_check_device(s)
+    held = not busy.query()
+    for t in threads:
+        t.join()
+    assert status == NOT_CONVERGED and L.pg_check_device(s) == 0
+    assert statuses == [0] * (n + 1) and [c.value for c in counts] == [14 * 18] * (n + 1)
+    assert held, "the words were not all taken for the whole time"
