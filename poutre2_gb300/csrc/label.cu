@@ -78,19 +78,9 @@ template <typename T, bool FLAT> __device__ __forceinline__ bool joined(T p, T q
 
 __device__ __forceinline__ void label_gave_up() { atomicCAS(&g_label_status, 0, (int)PG_ERR_CUDA); }
 
-__device__ __forceinline__ int32_t find_root(const int32_t *par, int32_t x) {
-  for (int it = 0; it < kLabelIters; ++it) {
-    const int32_t p = __ldcg(par + x);  // past L1: other CTAs write it
-    if (p == x) return x;
-    if (p < 0) break;  // a background pixel: never reached (only accepted pixels are joined)
-    x = p;
-  }
-  label_gave_up();
-  return x;
-}
-
-// The same, halving the path on the way: a parent replaced by its own parent stays an ancestor, so
-// later walks through the same tile roots are short (border unions of 2048^2 blobs: 20 -> 14 us).
+// Loads go past L1 (other CTAs write).  A parent replaced by its own parent stays an ancestor, so later walks through
+// the same tile roots are short (border unions of 2048^2 blobs: 20 -> 14 us).  A background pixel (parent < 0) is never
+// reached: only accepted pixels are joined.
 __device__ __forceinline__ int32_t find_halving(int32_t *par, int32_t x) {
   for (int it = 0; it < kLabelIters; ++it) {
     const int32_t p = __ldcg(par + x);
@@ -131,8 +121,30 @@ template <typename T> __device__ __forceinline__ T shfl_up(T v, int d) {
   else return __shfl_up_sync(0xffffffffu, v, d);
 }
 
-// STACKED: tiles of several slices.
-template <typename T, bool FLAT, bool STACKED>
+// A pixel as its row's equalities are tested.  Doubles as integers, for the double-precision pipe compares 32 of them in
+// 16 cycles or more (flat zones of 334 x 1120 f64: 22000 of a tile's 80000 cycles): equal bits mean equal values but for
+// the two zeros, which become one, and NaN, which equals nothing (key_nan).
+template <typename T> struct KeyOf { using type = T; };
+template <> struct KeyOf<double> { using type = int64_t; };
+template <typename T> using Key = typename KeyOf<T>::type;
+template <typename T> __device__ __forceinline__ Key<T> key_of(T v) {
+  if constexpr (std::is_same_v<T, double>) {
+    const int64_t b = __double_as_longlong(v);
+    return (b << 1) == 0 ? 0 : b;
+  } else {
+    return v;
+  }
+}
+template <typename T> __device__ __forceinline__ bool key_nan(Key<T> k) {
+  if constexpr (std::is_same_v<T, double>) return (k & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+  else return false;
+}
+
+// FULL: the form that waits less -- many runs of a chunk (noise, vertical segments) are handled four at a time, and the
+// pointer jumping ends with the first turn that moves nothing -- and that takes several slices a tile.  Where there
+// are tiles enough to hide the waits its longer code costs 3 % (binary 2048^2: 75 us without it, 77 with; flat zones
+// of 512^2 100 without, 86 with; 28 x 3 x 199 along z 100, 51).
+template <typename T, bool FLAT, bool FULL>
 __global__ void __launch_bounds__(kLThreads) k_label_tile(const T *__restrict__ in, int32_t *__restrict__ par,
                                                           unsigned *__restrict__ roots, LabelGeom g) {
   // masks of the chunks: chunk id = chunk column * tile rows + row, so the chunk above is id - 1.
@@ -147,26 +159,26 @@ __global__ void __launch_bounds__(kLThreads) k_label_tile(const T *__restrict__ 
   const uint32_t tile = blockIdx.x, tiles_x = (uint32_t)g.tiles_x, tiles_y = (uint32_t)g.tiles_y;
   const int nx = (int)g.nx;  // the image has less than 2^31 pixels: its indices are 32-bit
   const int x0 = (int)(tile % tiles_x) << g.log_tw, y0 = (int)(tile / tiles_x % tiles_y) << log_th;
-  const int ny = (int)g.ny, z0 = (int)(tile / tiles_x / tiles_y) * (STACKED ? g.slices : 1);
+  const int ny = (int)g.ny, z0 = (int)(tile / tiles_x / tiles_y) * (FULL ? g.slices : 1);
   const int row0 = z0 * ny + y0;  // first row, slices stacked
   const int w = min(tw, nx - x0);  // the tile inside the image
-  const int h = STACKED ? min(g.slices, (int)g.nz - z0) * ny : min(th, ny - y0);
+  const int h = FULL && g.slices > 1 ? min(g.slices, (int)g.nz - z0) * ny : min(th, ny - y0);
   const int base = row0 * nx + x0;
   const T *src = in + base;
   const bool hor = (g.edges & E_L) != 0, ver = (g.edges & E_U) != 0, eul = (g.edges & E_UL) != 0,
              eur = (g.edges & E_UR) != 0;
 
   // pixel c of row r, and (lanes 0 and 31) the pixel beside the chunk, if in the tile
-  auto load = [&](int r, int c, T &v, T &e) {
+  auto load = [&](int r, int c, Key<T> &v, Key<T> &e) {
     const int ce = lane == 0 ? c - 1 : c + 1;
     const T *q = src + r * nx;
     const bool row = r < h;
-    v = (row && c < w) ? q[c] : T(0);
-    e = (FLAT && row && (lane == 0 || lane == 31) && (unsigned)ce < (unsigned)w) ? q[ce] : T(0);
+    v = (row && c < w) ? key_of(q[c]) : Key<T>(0);
+    e = (FLAT && row && (lane == 0 || lane == 31) && (unsigned)ce < (unsigned)w) ? key_of(q[ce]) : Key<T>(0);
   };
   // ---- masks: a warp walks down its chunks
   constexpr int AT = FLAT ? 8 : 16;        // chunks whose loads go together
-  T pv = T(0), pe = T(0), nv[AT], ne[AT];  // pv, pe: the row above
+  Key<T> pv = 0, pe = 0, nv[AT], ne[AT];  // pv, pe: the row above
   if (FLAT && ((warp * 32) & (th - 1)) != 0)
     load(((warp * 32) & (th - 1)) - 1, ((warp * 32) >> log_th) * 32 + lane, pv, pe);
 #pragma unroll 1
@@ -179,16 +191,23 @@ __global__ void __launch_bounds__(kLThreads) k_label_tile(const T *__restrict__ 
 #pragma unroll
     for (int k = 0; k < AT; ++k) {
       const int id = warp * 32 + k0 + k;
-      const T v = nv[k], e = ne[k];
+      const Key<T> v = nv[k], e = ne[k];
       unsigned m0, m1, m2 = 0u, m3 = 0u;
       if constexpr (FLAT) {
-        T vl = shfl_up(v, 1), ul = shfl_up(pv, 1), ur = shfl_dn(pv, 1);
+        Key<T> vl = shfl_up(v, 1), ul = shfl_up(pv, 1), ur = shfl_dn(pv, 1);
         if (lane == 0) { vl = e; ul = pe; }
         if (lane == 31) ur = pe;
         m0 = __ballot_sync(0xffffffffu, v == vl);
         m1 = __ballot_sync(0xffffffffu, v == pv);
         m2 = __ballot_sync(0xffffffffu, v == ul);
         m3 = __ballot_sync(0xffffffffu, v == ur);
+        if constexpr (std::is_same_v<T, double>) {
+          const unsigned num = ~__ballot_sync(0xffffffffu, key_nan<T>(v));
+          m0 &= num;
+          m1 &= num;
+          m2 &= num;
+          m3 &= num;
+        }
         pv = v;
         pe = e;
       } else {
@@ -210,7 +229,7 @@ __global__ void __launch_bounds__(kLThreads) k_label_tile(const T *__restrict__ 
   // ---- runs: thread t owns chunk t
   const int id = threadIdx.x, r = id & (th - 1), cx = id >> log_th;
   const bool has_left = cx > 0, has_right = (cx + 1) * 32 < tw;      // neighbour chunks of the tile
-  const bool has_up = STACKED ? (unsigned)r % (unsigned)ny != 0u : r > 0;  // no edge up from a slice's first row
+  const bool has_up = FULL ? (unsigned)r % (unsigned)ny != 0u : r > 0;  // no edge up from a slice's first row
   const int l0 = (r << g.log_tw) + cx * 32;  // local raster index of the chunk's first pixel
   unsigned L, U = 0u, UL = 0u, UR = 0u, acc;
   {
@@ -285,15 +304,39 @@ __global__ void __launch_bounds__(kLThreads) k_label_tile(const T *__restrict__ 
   }
   __syncthreads();
   // pointer jumping: a link goes up a row or left a chunk, so six doublings flatten the usual tree
-  // (what is deeper still is walked by find_root).  Roots stay where they are (in noise nearly every run is one).
+  // (what is deeper still is walked by find).  Roots stay where they are (in noise nearly every run is one).
   volatile int32_t *vp = s_p;
 #pragma unroll 1
   for (int it = 0; it < 6; ++it) {
-    for (unsigned todo = hang; todo; todo &= todo - 1) {
-      const int i = ph(l0 + __ffs(todo) - 1);
-      vp[i] = vp[ph(vp[i])];
+    bool moved = false;
+    unsigned todo = hang;
+    // many runs in a chunk (vertical segments, noise): the loads of four go together
+    while (FULL && __popc(todo) > 6) {
+      int i[4], p[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k, todo &= todo - 1) {
+        i[k] = ph(l0 + __ffs(todo) - 1);
+        p[k] = vp[i[k]];
+      }
+      int q[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) q[k] = vp[ph(p[k])];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        moved |= q[k] != p[k];
+        vp[i[k]] = q[k];
+      }
     }
-    __syncthreads();
+    for (; todo; todo &= todo - 1) {
+      const int i = ph(l0 + __ffs(todo) - 1), p = vp[i], q = vp[ph(p)];
+      if (FULL) moved |= q != p;
+      vp[i] = q;
+    }
+    if constexpr (FULL) {
+      if (!__syncthreads_or(moved)) break;
+    } else {
+      __syncthreads();
+    }
   }
   // the edges left
   auto find = [&](int x) {
@@ -326,8 +369,39 @@ __global__ void __launch_bounds__(kLThreads) k_label_tile(const T *__restrict__ 
   }
   if (L) join(l0, run_of(id - th, 31));
   __syncthreads();
-  unsigned root_m = 0u;
-  for (unsigned todo = starts; todo; todo &= todo - 1) {
+  unsigned root_m = 0u, todo4 = starts;
+  while (FULL && __popc(todo4) > 6) {  // as above
+    int i[4], p[4];
+    unsigned bit[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      bit[k] = todo4 & (0u - todo4);
+      todo4 ^= bit[k];
+      i[k] = p[k] = l0 + __ffs(bit[k]) - 1;
+    }
+    bool more = true;
+    for (int it = 0; more; ++it) {
+      int q[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) q[k] = vp[ph(p[k])];
+      more = false;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        more |= q[k] != p[k];
+        p[k] = q[k];
+      }
+      if (more && it == kLabelIters) {
+        label_gave_up();
+        break;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      vp[ph(i[k])] = p[k];
+      if (p[k] == i[k]) root_m |= bit[k];
+    }
+  }
+  for (unsigned todo = todo4; todo; todo &= todo - 1) {
     const int l = l0 + __ffs(todo) - 1, p = find(l);
     vp[ph(l)] = p;
     if (p == l) root_m |= todo & (0u - todo);
@@ -418,39 +492,61 @@ __global__ void __launch_bounds__(kLThreads) k_label_border(const T *__restrict_
 
 // ------------------------------------------------------------------ numbering
 // Tile roots find their component's root; the bitmap keeps the components' roots, counted per segment.
+// PARTS threads a word, whose roots are followed four at a time: noise and the columns of vertical segments have up to
+// 32 tile roots a word, each a chain of L2 loads (12 x 10 x 363 along z: 40 us with a thread a word and one root after
+// the other, 12 with four threads; with few roots a word one thread is 1 us faster on 2048^2).
+template <int PARTS>
 __global__ void __launch_bounds__(kLThreads) k_label_flatten(int32_t *par, unsigned *__restrict__ roots,
                                                              int32_t *__restrict__ cnt, LabelGeom g, int64_t words,
                                                              int log_seg) {
-  int32_t own = 0;
-  const int64_t wi = (int64_t)blockIdx.x * kLThreads + threadIdx.x;
-  if (wi < words) {
-    const unsigned m = roots[wi];
-    unsigned keep = m;
-    if (m) {
-      const int64_t row = (uint32_t)wi / (uint32_t)g.words_x;
-      const int32_t i0 = (int32_t)(row * g.nx + (wi - row * g.words_x) * 32);
-      for (unsigned todo = m; todo;) {
-        // the loads of four roots go together (noise has nearly 32 a word: flat zones of 512^2 14 -> 6 us)
-        unsigned bit[4];
-        int32_t p[4];
+  const int64_t t = (int64_t)blockIdx.x * kLThreads + threadIdx.x, wi = t / PARTS;
+  const unsigned which = (unsigned)t % PARTS, part = PARTS == 1 ? ~0u : 0xffu << (8 * which);
+  const unsigned m = wi < words ? roots[wi] : 0u;
+  unsigned gone = 0u;
+  if (m & part) {
+    const int64_t row = (uint32_t)wi / (uint32_t)g.words_x;
+    const int32_t i0 = (int32_t)(row * g.nx + (wi - row * g.words_x) * 32);
+    for (unsigned todo = m & part; todo;) {
+      unsigned bit[4];
+      int32_t p[4];  // the pixel, then its ancestors; -1: no root here
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        bit[k] = todo & (0u - todo);
+        todo ^= bit[k];
+        p[k] = bit[k] ? i0 + __ffs(bit[k]) - 1 : -1;
+      }
+      bool more = true;
+      for (int it = 0; more; ++it) {
+        int32_t q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = p[k] >= 0 ? __ldcg(par + p[k]) : -1;
+        more = false;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          bit[k] = todo & (0u - todo);
-          todo ^= bit[k];
-          p[k] = bit[k] ? __ldcg(par + i0 + __ffs(bit[k]) - 1) : -1;
+          if (q[k] < 0 || q[k] == p[k]) continue;
+          p[k] = q[k];
+          more = true;
         }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int32_t i = i0 + __ffs(bit[k]) - 1;
-          if (p[k] < 0 || p[k] == i) continue;
-          keep ^= bit[k];
-          __stcg(par + i, find_root(par, p[k]));
+        if (more && it == kLabelIters) {
+          label_gave_up();
+          break;
         }
       }
-      if (keep != m) roots[wi] = keep;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int32_t i = i0 + __ffs(bit[k]) - 1;
+        if (p[k] < 0 || p[k] == i) continue;
+        gone |= bit[k];
+        __stcg(par + i, p[k]);
+      }
     }
-    own = __popc(keep);
   }
+  if constexpr (PARTS == 4) {
+    gone |= __shfl_xor_sync(0xffffffffu, gone, 1);
+    gone |= __shfl_xor_sync(0xffffffffu, gone, 2);
+  }
+  if (gone != 0u && which == 0) roots[wi] = m & ~gone;
+  int32_t own = __popc(m & ~gone & part);
   // a segment is a whole number of CTAs' words
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) own += __shfl_xor_sync(0xffffffffu, own, o);
@@ -629,7 +725,9 @@ pg_status label_t(const pg_image &in, const pg_image &out, unsigned edges, int64
   int64_t *o = static_cast<int64_t *>(out.data);
   const T *src = static_cast<const T *>(in.data);
   PG_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)nseg, s), "clear label counts");
-  if (g.slices > 1) k_label_tile<T, FLAT, true><<<(unsigned)tiles, kLThreads, 0, s>>>(src, par, roots, g);
+  // the forms that wait less for flat zones of few tiles and for columns of runs
+  const bool full = g.slices > 1 || (FLAT && tiles <= 2 * num_sms()) || !(edges & E_L);
+  if (full) k_label_tile<T, FLAT, true><<<(unsigned)tiles, kLThreads, 0, s>>>(src, par, roots, g);
   else k_label_tile<T, FLAT, false><<<(unsigned)tiles, kLThreads, 0, s>>>(src, par, roots, g);
   const int64_t n_rows = (edges & (E_U | E_UL | E_UR)) ? d.nz * (g.tiles_y - 1) * d.nx : 0;
   const int64_t n_cols = (edges & (E_L | E_UL | E_UR)) ? d.nz * d.ny * (g.tiles_x - 1) : 0;
@@ -638,7 +736,8 @@ pg_status label_t(const pg_image &in, const pg_image &out, unsigned edges, int64
   if (items > 0)
     k_label_border<T, FLAT><<<(unsigned)std::min<int64_t>(ceil_div(items, kLThreads), cap), kLThreads, 0, s>>>(
         src, par, g, n_rows, n_cols, n_z);
-  k_label_flatten<<<(unsigned)ceil_div(words, kLThreads), kLThreads, 0, s>>>(par, roots, cnt, g, words, log_seg);
+  if (full) k_label_flatten<4><<<(unsigned)ceil_div(4 * words, kLThreads), kLThreads, 0, s>>>(par, roots, cnt, g, words, log_seg);
+  else k_label_flatten<1><<<(unsigned)ceil_div(words, kLThreads), kLThreads, 0, s>>>(par, roots, cnt, g, words, log_seg);
   if (log_seg < 10) k_label_number<1><<<(unsigned)nseg, kLThreads, 0, s>>>(par, roots, cnt, g, words, log_seg, total);
   else k_label_number<4><<<(unsigned)nseg, kLThreads, 0, s>>>(par, roots, cnt, g, words, log_seg, total);
   const unsigned rg = (unsigned)ceil_div(n, 4 * kLThreads);
