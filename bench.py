@@ -542,7 +542,7 @@ def extra_measurements(dev, flush, only=None, cfg5_batch=64):
 
     def geodesy3d():
         # binary h-maxima (h = 10) of a 128^3 u8 volume (white noise, Gaussian sigma 2, rescaled),
-        # SECross3D: the iterated geodesic step of the volume route, poutre2 on one core beside it
+        # SECross3D: the resident bricks of the volume route, poutre2 on one core beside it
         from scipy.ndimage import gaussian_filter
         rng = np.random.default_rng(12)
         v = gaussian_filter(rng.standard_normal((128, 128, 128)), 2.0, mode="reflect", truncate=4.0)
@@ -551,7 +551,7 @@ def extra_measurements(dev, flush, only=None, cfg5_batch=64):
         o = torch.empty_like(x)
         for se in ("SECross3D",):
             ms = _time_ms(lambda se=se: geo.h_maxima_binary(x, 10, Common_NL_SE[se], o, check=False), flush, 5, 2)
-            kw = {"note": "includes the host reads of the change flag (every two brick launches)"}
+            kw = {"note": "one launch: the volume's bricks stay on the GPU"}
             try:
                 from oracle import ref
                 if ref.available():

@@ -366,17 +366,22 @@ PG_API pg_status pg_reconstruction_noalloc(int32_t type, const pg_image *marker,
 PG_API pg_status pg_check_device(pg_stream_t stream);
 
 /* Test hooks (no counterpart in the reference), for tests of the failure paths without a GPU fault.
- * pg_debug_set_limits: max_rounds > 0 caps the reconstruction's rounds (round kernel) or visits per
- * tile (worklist kernel), wait_ns > 0 sets the limit of every bounded device wait of the
- * reconstruction kernels launched afterwards (default 4 s); a run that reaches either gives up and
- * pg_check_device returns PG_ERR_NOT_CONVERGED.  0 restores the default.  Process-wide.
+ * pg_debug_set_limits: max_rounds > 0 caps the reconstruction's rounds (round kernel), its visits per
+ * tile on average (worklist kernel) or those of any one tile or brick (resident kernels), wait_ns > 0
+ * sets the limit of every bounded device wait of the reconstruction kernels launched afterwards
+ * (default 4 s; a resident tile's wait for work counts from the last progress of any tile); a run that
+ * reaches either gives up and pg_check_device returns PG_ERR_NOT_CONVERGED.  0 restores the default.
+ * Process-wide.
  * pg_debug_fail_allocations: the next n temporary allocations fail (PG_ERR_OUT_OF_MEMORY). */
 PG_API pg_status pg_debug_set_limits(int32_t max_rounds, int64_t wait_ns);
 PG_API pg_status pg_debug_fail_allocations(int32_t n);
 
 /* Passes of the last completed reconstruction on the current device (diagnostics; synchronises
- * the device): for the shared-memory tile kernel the rounds of tile visits, for the worklist kernel
- * (pixels of at most 4 bytes) the tile visits divided by the number of tiles, rounded up. */
+ * the device): for the shared-memory tile kernel (8-byte pixels, the allocation-free entry) the rounds
+ * of tile visits, for the resident kernels (images and volumes of 1- or 2-byte pixels whose tiles all
+ * stay on the GPU) the most visits of any one tile, for the worklist kernel (other images of pixels of
+ * at most 4 bytes) the tile visits divided by the number of tiles, rounded up.  Other volumes leave it
+ * as it was. */
 PG_API int32_t pg_last_reconstruction_rounds(void);
 
 #ifdef __cplusplus

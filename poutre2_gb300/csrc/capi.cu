@@ -174,6 +174,7 @@ static pg_status repeat_small(const pg_image &in, int se, int iter, const pg_ima
 //     window kernel (window.cu) at once: 3x3 u8 19 / 35, X segment f32 27 / 37; below 3 Mpixel (4-byte
 //     pixels: 8, f32 2052 x 1674 13 / 11) its fixed cost weighs more (500 x 501: 8 / 6);
 //   k = 7, 15, 31 on 16-byte rows: the TMA tiles (Y segments diag.cu, boxes rect.cu): 31x31 u16 20 / 51;
+//   (images so narrow that a window tile is mostly empty: the kernels below, window_narrow in window.cu)
 //   rectangles: the window kernel: u8 21x21 33 / 44, f32 11x11 53 / 95, ragged u8 29 / 120; where rows are
 //     whole words the two line passes win from hy + hx = 45 on (u8 45x45 46 / 46, 63x63 50 / 57);
 //   X segments: the word tiles (line_w.cu), where rows are whole words (u8 k = 10 20 / 22, u16 27 / 31), but

@@ -23,7 +23,10 @@
 // 0.80 ms on a thresholded 2048^2 u8 image, nearly all of it in long chains of dependent loads
 // contending for the same few roots; a tile's chains are in shared memory, and one pixel in forty
 // reaches global memory.  2048^2 u8 binary: tile 25 us,
-// border 14, flatten 6, number 4, resolve 11; 77 us a call with the count's read back, against 800.
+// border 11, flatten 6, number 5, resolve 11; 75 us a call with the count's read back, against 800.  Where
+// nearly every pixel is a component of its own there are no such chains, and small images of that kind
+// are what the tiles cost most on: flat zones of 512^2 noise 56 us against 53, of 605 x 216 textured by
+// threes 71 against 42 (512^2 blobs 52 against 188).
 // The floor (input read, labels written) is 5.6 us; the tile pass is bound by the dependent shared-memory
 // loads of the runs (40 % of the issue slots), border and flatten by the L2 latency of their chains.
 //
@@ -130,7 +133,7 @@ template <typename T> using Key = typename KeyOf<T>::type;
 template <typename T> __device__ __forceinline__ Key<T> key_of(T v) {
   if constexpr (std::is_same_v<T, double>) {
     const int64_t b = __double_as_longlong(v);
-    return (b << 1) == 0 ? 0 : b;
+    return (b & 0x7fffffffffffffffll) == 0 ? 0 : b;
   } else {
     return v;
   }

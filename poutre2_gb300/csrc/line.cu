@@ -193,8 +193,11 @@ pg_status launch_line(const pg_image &in, const pg_image &out, int dy, int dx, i
   else kmax = std::min(d.ny, d.nx) - 1;
   const int64_t k = std::min<int64_t>(half, std::max<int64_t>(kmax, 0));
   if (k >= 1 && k <= (1 << 20)) {
-    // Y and diagonal segments: the TMA tiles or the register streams where they have the length, else the
-    // window kernel (4096^2, us, with / without it: u8 45 degrees k = 10 26 / 45, f32 43 / 104; ragged 2999 x 4001 u8 Y
+    // Y and diagonal segments: the TMA tiles or the register streams where they have the length (half lengths 1, 2, 3,
+    // 7, 15, 31 on whole-word rows; us, stream / window, rows that miss the 16 bytes of the TMA tiles: Y k = 7, 15, 31 f32
+    // 3000 x 3501 20 / 25, 22 / 29, 31 / 38, u16 8000 x 8002 50 / 76, 57 / 89, 75 / 123, u8 2999 x 4004 13 / 17, 16 / 19, 17 / 23; 45 degrees
+    // f32 3000 x 3501 23 / 25, 27 / 29, 35 / 39, but u16 2999 x 4002 k = 31 44 / 31; and below a megapixel the window is the
+    // shorter launch: 512 x 501 f32 Y k = 7 8 / 6), else the window kernel (4096^2, us, with / without it: u8 45 degrees k = 10 26 / 45, f32 43 / 104; ragged 2999 x 4001 u8 Y
     // 22 / 68, 45 degrees 21 / 90).  Y segments of whole-word rows keep the word tiles of line_w.cu where those are the
     // faster: u8 between 1.5 and 20 Mpixel (k = 4 to 30: 3735 x 7360 23 / 27, 1975 x 628 8 / 9, but 1520 x 5856 21 / 15, 903 x
     // 2900 11 / 9; from k = 36 on up to 7: 5190 x 3584 k = 60 44 / 54) and long ones of small images (k above 10; u16

@@ -244,8 +244,8 @@ bool try_line_stream(const pg_image &in, const pg_image &out, int dy, int dx, in
   if (H < 1 || H > (1 << 30) || W > (1 << 29) || ceil_div(H, 32) > 65535) return false;
   // the vertical kernel and the 1-/2-byte diagonal kernel move whole 32-bit words; the 4-byte
   // diagonal one single pixels
-  // u8 diagonals of 63 pixels: the word kernel's register window (196 registers) leaves too few
-  // warps; the staircase tiles of line_w.cu measured faster there (54 vs 68 us on 4096^2)
+  // u8 diagonals of 63 pixels: the word kernel's register window (196 registers) leaves too few warps (68 us on
+  // 4096^2 against 54 on the staircase tiles of line_w.cu); the window kernel takes them (23 on 2999 x 4004)
   if (dx != 0 && es == 1 && k > 15) return false;
   if ((W * es) % 4 != 0) return false;
   if ((reinterpret_cast<uintptr_t>(in.data) | reinterpret_cast<uintptr_t>(out.data)) % 4 != 0) return false;

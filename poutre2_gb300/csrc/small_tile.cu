@@ -192,9 +192,8 @@ __global__ void __launch_bounds__(kSTThreads) k_small2d_tile(const __grid_consta
 }
 
 // The same tile of 64 words by kST2QRows rows with a thread per 16-byte quad of words and
-// kST2QRows / 8 rows: each box row is read as one 16-byte load plus the two neighbouring words, each
-// u8 word split once (not three times, as the centre and as each neighbour's neighbour), and the
-// results stored 16 bytes at a time.
+// kST2QRows / 8 rows: each box row is read as one 16-byte load plus the two neighbouring words (not three
+// words per word), and the results stored 16 bytes at a time.
 template <typename T, bool SUP, int SHAPE>
 __global__ void __launch_bounds__(kST2QThreads) k_small2d_quad(const __grid_constant__ CUtensorMap tmap,
                                                             uint32_t *__restrict__ out, int H, int Wn) {
