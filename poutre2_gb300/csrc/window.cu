@@ -692,6 +692,15 @@ bool try_window(const pg_image &in, const pg_image &out, int64_t hy, int64_t hx,
   }
 }
 
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return status != cudaStreamCaptureStatusNone;
+}
+
 bool try_chords(const pg_image &in, const pg_image &out, const int32_t *offsets, int n, bool dilate, cudaStream_t s,
                 pg_status *st) {
   const int es = elem_size(in.ptype);
@@ -704,7 +713,9 @@ bool try_chords(const pg_image &in, const pg_image &out, const int32_t *offsets,
   int span = 0, longest = 1;
   if (!make_chords(offsets, n, in.rank, 4 / es, es == 4 ? 32 : 64, t, span, longest)) return false;
   const ChordTiles c = chord_tiles(in, out, longest);
-  if (!chords_win(t, c, d, es, n)) return false;
+  // While the stream captures, the chords whatever they cost: their list goes by value into the graph, where a copy of
+  // the gather's would read this call's host memory at every launch of the graph.
+  if (!chords_win(t, c, d, es, n) && !capturing(s)) return false;
   switch (in.ptype) {
     case PG_PTYPE_U8: *st = dilate ? chords_t<uint8_t, true>(in, out, t, c, span, s) : chords_t<uint8_t, false>(in, out, t, c, span, s); return true;
     case PG_PTYPE_U16: *st = dilate ? chords_t<uint16_t, true>(in, out, t, c, span, s) : chords_t<uint16_t, false>(in, out, t, c, span, s); return true;

@@ -46,6 +46,41 @@ def test_volumes(dt):
         _check(rng.integers(0, 250, shape).astype(dt), ball)
 
 
+def test_a_captured_list_outlives_the_call():
+    # a small image, whose list would be gathered: in a graph it goes by value
+    import ctypes
+
+    from poutre2_gb300 import _lib
+    from poutre2_gb300.image import descriptor
+    L, driver = _lib.load(), ctypes.CDLL("libcuda.so.1")
+    offsets = LISTS["disk"]
+    a = np.random.default_rng(5).integers(0, 250, (50, 60)).astype(np.uint8)
+    x = torch.from_numpy(a).cuda()
+    out = torch.empty_like(x)
+    dx, do = descriptor(x), descriptor(out)
+    flat = (ctypes.c_int32 * (2 * len(offsets)))(*[v for o in offsets for v in o])
+    stream = torch.cuda.Stream()
+    s = ctypes.c_void_p(stream.cuda_stream)
+    torch.cuda.synchronize()
+    assert L.pg_dilate_nl(ctypes.byref(dx), flat, len(offsets), ctypes.byref(do), s) == 0  # the kernels are loaded
+    stream.synchronize()
+    assert driver.cuStreamBeginCapture_v2(s, 0) == 0
+    assert L.pg_dilate_nl(ctypes.byref(dx), flat, len(offsets), ctypes.byref(do), s) == 0
+    graph, ready = ctypes.c_void_p(), ctypes.c_void_p()
+    assert driver.cuStreamEndCapture(s, ctypes.byref(graph)) == 0 and graph.value
+    assert driver.cuGraphInstantiateWithFlags(ctypes.byref(ready), graph, ctypes.c_ulonglong(0)) == 0
+    ctypes.memset(flat, 0, ctypes.sizeof(flat))
+    junk = [np.full(n, 7, np.int32) for n in range(16, 4096, 16)]  # the call's host memory is somebody else's now
+    for _ in range(2):
+        out.zero_()
+        torch.cuda.synchronize()
+        assert driver.cuGraphLaunch(ready, s) == 0
+        stream.synchronize()
+        np.testing.assert_array_equal(out.cpu().numpy(), oracle.erode_dilate_nl(a, offsets, True))
+    assert junk[0][0] == 7
+    assert driver.cuGraphExecDestroy(ready) == 0 and driver.cuGraphDestroy(graph) == 0
+
+
 def test_more_offsets_than_a_list_may_hold():
     from poutre2_gb300 import llm
     from poutre2_gb300._lib import PoutreError
